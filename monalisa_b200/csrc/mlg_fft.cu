@@ -10,6 +10,8 @@
 #include <vector>
 
 #include "mlg_fft_kernels.cuh"
+#include "mlg_fft_reg.cuh"
+#include "mlg_fft_reg_lengths.h"
 
 namespace mlg {
 
@@ -18,6 +20,11 @@ bool tma_passes_enabled() {
     const char* e = std::getenv("MLG_FFT_TMA");
     return !(e && std::strcmp(e, "0") == 0);
   }();
+  return on;
+}
+
+bool register_passes_default() {
+  static const bool on = std::getenv("MLG_FFT_TMA") == nullptr;
   return on;
 }
 
@@ -118,8 +125,34 @@ int fft_axis_init(int N, FftAxisPlan& a) {
     const double ang = -2.0 * M_PI * (double)j / (double)N;
     t[j] = make_float2((float)std::cos(ang), (float)std::sin(ang));
   }
-  MLG_CUDA(cudaMalloc(&a.tw, sizeof(float2) * N));
-  MLG_CUDA(cudaMemcpy(a.tw, t.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+  switch (N) {
+#define X(LEN, A, B, MAIN) \
+  case LEN:                \
+    a.rA = A;              \
+    a.rB = B;              \
+    break;
+    MLG_REG_ALL(X)
+#undef X
+    default: break;
+  }
+  if (a.rA) {  // the register passes' tables: W_N^(n2 k1), conjugated for the inverse
+    t.resize(3 * (size_t)N);
+    for (int dir = 0; dir < 2; ++dir) {
+      const int n1s = dir ? a.rB : a.rA;
+      float2* u = t.data() + (size_t)(dir + 1) * N;
+      for (int n2 = 0; n2 < N / n1s; ++n2)
+        for (int k1 = 0; k1 < n1s; ++k1) {
+          const float2 w = t[(size_t)n2 * k1];  // n2 k1 < N
+          u[(size_t)n2 * n1s + k1] = make_float2(w.x, dir ? -w.y : w.y);
+        }
+    }
+  }
+  MLG_CUDA(cudaMalloc(&a.tw, sizeof(float2) * t.size()));
+  MLG_CUDA(cudaMemcpy(a.tw, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice));
+  if (a.rA) {
+    a.rtw[0] = a.tw + N;
+    a.rtw[1] = a.tw + 2 * (size_t)N;
+  }
   return MLG_OK;
 }
 
@@ -129,7 +162,31 @@ void fft_axis_free(FftAxisPlan& a) {
 }
 
 int fft_pass_blocks(const FftAxisPlan& a, const PassDesc& d) {
-  return blocks_for(d, lines_per_cta(a, d.C, PassMode::kNakatshaOut));
+  return std::max(kRegMaxBlocks, blocks_for(d, lines_per_cta(a, d.C, PassMode::kNakatshaOut)));
+}
+
+int fft_reg_group_0(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+int fft_reg_group_1(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+int fft_reg_group_2(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+int fft_reg_group_3(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+int fft_reg_group_4(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+int fft_reg_group_5(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+int fft_reg_group_6(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+int fft_reg_group_7(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+int fft_reg_group_8(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+int fft_reg_group_9(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+
+// The pass's register kernel; *done stays false where there is none.
+static int fft_reg_pass(const FftAxisPlan& a, PassMode mode, const PassDesc& d, int* n_partial, cudaStream_t s,
+                        bool* done) {
+  using Fn = int (*)(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+  static const Fn kGroups[] = {fft_reg_group_0, fft_reg_group_1, fft_reg_group_2, fft_reg_group_3, fft_reg_group_4, fft_reg_group_5, fft_reg_group_6, fft_reg_group_7, fft_reg_group_8, fft_reg_group_9};
+  *done = false;
+  for (Fn f : kGroups) {
+    const int st = f(a, mode, d, n_partial, s, done);
+    if (st != MLG_OK || *done) return st;
+  }
+  return MLG_OK;
 }
 
 int fft_pass(const FftAxisPlan& a, PassMode mode, const PassDesc& d, int* n_partial, cudaStream_t s) {
@@ -138,6 +195,12 @@ int fft_pass(const FftAxisPlan& a, PassMode mode, const PassDesc& d, int* n_part
   const int L = lines_per_cta(a, d.C, mode);
   MLG_CHECK((size_t)a.N * L * d.C * sizeof(float2) <= 200 * 1024,
             "FFT line of %d points x %d coils exceeds shared memory", a.N, d.C);
+  if (d.reg && !d.dry && a.rA > 0 && mode != PassMode::kGutIn) {
+    bool done = false;
+    if (n_partial) *n_partial = 0;
+    MLG_TRY(fft_reg_pass(a, mode, d, n_partial, s, &done));
+    if (done) return MLG_OK;
+  }
   if (n_partial) *n_partial = mode == PassMode::kNakatshaOut && d.partial ? blocks_for(d, L) : 0;
   switch (mode) {
     case PassMode::kShannaIn:

@@ -24,6 +24,11 @@ struct FftAxisPlan {
   int N = 0, N1 = 0, N2 = 0;  // N = N1 * N2, both <= 32
   bool fast = false;          // templated power-of-two path
   float2* tw = nullptr;       // exp(-2 pi i j / N), j < N (device)
+  // register passes (mlg_fft_reg.cuh), for lengths that have them: the split
+  // N = rA * rB (0: none) and the step-A twiddles [n2][k1] of the forward
+  // (N1 = rA) and inverse (N1 = rB) transforms (in tw's allocation)
+  int rA = 0, rB = 0;
+  float2* rtw[2] = {nullptr, nullptr};
 };
 
 struct PassDesc {
@@ -80,6 +85,12 @@ struct PassDesc {
   int h_len = 1;
   int h_len_out = 0;  // with both in_half and out_half: the output's h_len (0: h_len)
   unsigned* out_absmax = nullptr;
+  // register passes (mlg_fft_reg.cuh) where the axis and the pass's shape
+  // have one; tmask / out_tmask: in_lmask / out_lmask regrouped for them (bit
+  // j of word [line][m] = row m + rA j)
+  int reg = 0;
+  const uint32_t* tmask = nullptr;
+  const uint32_t* out_tmask = nullptr;
   // check only: MLG_OK when a kernel would run the pass with every field
   // above honoured, MLG_ERR_UNSUPPORTED otherwise; nothing is launched
   int dry = 0;
@@ -100,13 +111,16 @@ int fft_wait_status(int* word, cudaStream_t s);
 // Whether the TMA passes may run at all (MLG_FFT_TMA=0 turns them off for
 // every plan; otherwise PassDesc::tma_slots decides per pass).
 bool tma_passes_enabled();
+// Whether plans start on the register passes: yes, unless MLG_FFT_TMA asks for
+// the shared-memory passes with (1) or without (0) the TMA unit.
+bool register_passes_default();
 
 int fft_axis_init(int N, FftAxisPlan& a);
 void fft_axis_free(FftAxisPlan& a);
 // Launches one pass; *n_partial receives the CTA count when partial sums are
 // written (kNakatshaOut).
 int fft_pass(const FftAxisPlan& a, PassMode mode, const PassDesc& d, int* n_partial, cudaStream_t s);
-// CTA count of a pass (for partial-sum buffer sizing).
+// An upper bound of a pass's CTA count (for partial-sum buffer sizing).
 int fft_pass_blocks(const FftAxisPlan& a, const PassDesc& d);
 
 }  // namespace mlg

@@ -48,6 +48,7 @@ static void box_strides(const int e[3], int C, long long st[3]) {
 static void set_masked_store(const mlg_plan_s* p, PassDesc& pd) {
   if (p->fwd_masked_store && p->gu_covered && p->line_mask) {
     pd.out_lmask = p->line_mask;
+    pd.out_tmask = p->tmask;
     pd.lmask_words = p->line_mask_words;
   }
 }
@@ -71,6 +72,7 @@ static int forward_pass(mlg_plan_s* p, int ax, const float2* x, bool x_per_coil,
   pd.C = C;
   pd.wait_err = p->wait_err;
   pd.tma_slots = p->pass_buffers;
+  pd.reg = p->reg_passes;
   pd.dry = dry ? 1 : 0;
   if (half) {
     pd.h_amax = p->mix_amax;
@@ -177,6 +179,7 @@ static int inverse_pass(mlg_plan_s* p, int ax, const float2* y, const float* HY,
   pd.C = C;
   pd.wait_err = p->wait_err;
   pd.tma_slots = p->pass_buffers;
+  pd.reg = p->reg_passes;
   pd.dry = dry ? 1 : 0;
   if (half) {
     pd.h_amax = p->mix_amax + 1;
@@ -187,6 +190,7 @@ static int inverse_pass(mlg_plan_s* p, int ax, const float2* y, const float* HY,
   if (p->adjoint_mode == kAdjMasked && ax == d - 1) {
     pd.in_mask = p->Gut_s.nz_mask;
     pd.in_lmask = p->line_mask;
+    pd.tmask = p->tmask;
     pd.lmask_words = p->line_mask_words;
     pd.cell_stride[0] = 1;
     pd.cell_stride[1] = p->N[0];
@@ -437,6 +441,25 @@ __global__ void line_mask_kernel(const uint32_t* __restrict__ nz, int du, int dv
   }
 }
 
+// The same bits regrouped for the register passes: bit j of word m of a line
+// = cell m + A j of it, m < A (the rows one thread of such a pass loads or
+// stores).
+__global__ void line_tmask_kernel(const uint32_t* __restrict__ lm, long long lines, int LW, int Nax, int A,
+                                  uint32_t* __restrict__ tm) {
+  const long long total = lines * A;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+       i += (long long)gridDim.x * blockDim.x) {
+    const long long line = i / A;
+    const int m = (int)(i - line * A);
+    uint32_t w = 0;
+    for (int j = 0; m + A * j < Nax; ++j) {
+      const int n = m + A * j;
+      w |= ((lm[line * LW + (n >> 5)] >> (n & 31)) & 1u) << j;
+    }
+    tm[i] = w;
+  }
+}
+
 // 1 in *miss when a Gu column (a grid cell Gu reads) is not an occupied cell
 // of Gut's occupancy bits.
 __global__ void cover_check_kernel(const int* __restrict__ col, long long nnz, const uint32_t* __restrict__ nz,
@@ -475,11 +498,18 @@ static int build_line_mask(mlg_plan_s* p, cudaStream_t s) {
   const int v = ax == 2 ? 1 : 2;
   const int LW = ((p->N[ax] + 31) / 32 + 3) / 4 * 4;
   const long long total = (long long)du * dv * LW;
-  MLG_CUDA(cudaMalloc(&p->line_mask, sizeof(uint32_t) * (size_t)total));
+  const long long lines = (long long)du * dv;
+  const int A = p->ax[ax].rA;
+  MLG_CUDA(cudaMalloc(&p->line_mask, sizeof(uint32_t) * (size_t)(total + lines * A)));
   p->line_mask_words = LW;
   line_mask_kernel<<<ew_grid(total), kEwThreads, 0, s>>>(p->Gut_s.nz_mask, du, dv, cs[0], cs[v], cs[ax], p->N[ax], LW,
                                                          p->line_mask);
   MLG_LAUNCHED();
+  if (A) {
+    p->tmask = p->line_mask + total;
+    line_tmask_kernel<<<ew_grid(lines * A), kEwThreads, 0, s>>>(p->line_mask, lines, LW, p->N[ax], A, p->tmask);
+    MLG_LAUNCHED();
+  }
   return MLG_OK;
 }
 
@@ -616,6 +646,7 @@ static int plan_create_impl(int imDim, const int* N_u, const int* n_u, int nCh, 
     return bail(st);
   if (Gut && (st = csr_sign_copy(*Gut, true, imDim, p->N, 1.0f, p->Gut_s, s)) != MLG_OK) return bail(st);
   if (Gut && (nCh % 2) == 0 && nCh / 2 <= 16 && (st = csr_build_records(p->Gut_s, s)) != MLG_OK) return bail(st);
+  p->reg_passes = register_passes_default() ? 1 : 0;
   p->gut_records = p->Gut_s.ord_rec ? 1 : 0;  // measured faster on c2 (0.607 vs 0.671 ms)
   if ((st = build_line_mask(p, s)) != MLG_OK) return bail(st);
   if ((st = check_gu_covered(p, s)) != MLG_OK) return bail(st);

@@ -41,6 +41,9 @@ struct mlg_plan_s {
   // tables, for kAdjMasked)
   uint32_t* line_mask = nullptr;
   int line_mask_words = 0;
+  // the same bits regrouped for the register passes (PassDesc::tmask; in
+  // line_mask's allocation)
+  uint32_t* tmask = nullptr;
   double* scalars = nullptr;      // solver scalars (device)
   int* wait_err = nullptr;        // the device's pass wait flag (fft_wait_word, not owned)
   // kernel variants chosen per plan (mlg_plan_autotune_variants): line-FFT
@@ -50,6 +53,9 @@ struct mlg_plan_s {
   // forward pass storing only the 32-row chunks that hold cells Gu reads
   // (fwd_masked_store = 1; allowed when gu_covered: every Gu column is an
   // occupied cell of the line masks, checked once at plan creation)
+  // register passes (mlg_fft_reg.cuh; the default) in place of either, for
+  // the pass shapes that have one
+  int reg_passes = 0;
   int pass_buffers = 2;
   int gut_records = 0;
   int fwd_masked_store = 0;

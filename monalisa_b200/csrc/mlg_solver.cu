@@ -510,7 +510,9 @@ extern "C" int mlg_plan_set_variant(mlg_plan_t p, int pass_buffers, int gut_reco
   MLG_CHECK(!gut_records || p->Gut_s.ord_rec, "this plan has no Gut row records (masked adjoint, even coil count)");
   MLG_CHECK(!fwd_masked_store || p->gu_covered,
             "this plan cannot mask its forward stores (no line masks, or a Gu column outside Gut's occupied cells)");
-  if (p->pass_buffers != pass_buffers || p->gut_records != gut_records || p->fwd_masked_store != fwd_masked_store) {
+  if (p->reg_passes || p->pass_buffers != pass_buffers || p->gut_records != gut_records ||
+      p->fwd_masked_store != fwd_masked_store) {
+    p->reg_passes = 0;  // the named passes run
     p->pass_buffers = pass_buffers;
     p->gut_records = gut_records;
     p->fwd_masked_store = fwd_masked_store;
@@ -518,6 +520,24 @@ extern "C" int mlg_plan_set_variant(mlg_plan_t p, int pass_buffers, int gut_reco
     p->cg_graph = nullptr;
     p->cg_graph_x = nullptr;
   }
+  return MLG_OK;
+}
+
+extern "C" int mlg_plan_set_register_passes(mlg_plan_t p, int on) {
+  MLG_CHECK(p, "NULL plan");
+  MLG_CHECK(on == 0 || on == 1, "register passes: 0 or 1");
+  if (p->reg_passes != on) {
+    p->reg_passes = on;
+    if (p->cg_graph) cudaGraphExecDestroy(p->cg_graph);  // captured with the other kernels
+    p->cg_graph = nullptr;
+    p->cg_graph_x = nullptr;
+  }
+  return MLG_OK;
+}
+
+extern "C" int mlg_plan_get_register_passes(mlg_plan_t p, int* on) {
+  MLG_CHECK(p && on, "NULL argument");
+  *on = p->reg_passes;
   return MLG_OK;
 }
 
@@ -530,7 +550,7 @@ extern "C" int mlg_plan_get_variant(mlg_plan_t p, int* pass_buffers, int* gut_re
 }
 
 // Times the kernel variants of the plan's current adjoint strategy and keeps
-// the fastest: ms[0..2] = forward + adjoint with TMA passes over 2 / 3
+// the fastest (the register passes included): ms[0..2] = forward + adjoint with TMA passes over 2 / 3
 // buffers and with cp.async passes (masked forward stores where the plan
 // allows them), ms[3..4] = adjoint with Gut from the CSR / from row records,
 // ms[5] = forward + adjoint storing every chunk of the grid, at the chosen
@@ -562,7 +582,8 @@ extern "C" int mlg_plan_autotune_variants(mlg_plan_t p, int reps, double* ms) {
     cudaEventElapsedTime(&v, a, b);
     return (double)v / reps;
   };
-  const int buf0 = p->pass_buffers, rec0 = p->gut_records, mask0 = p->fwd_masked_store;
+  const int buf0 = p->pass_buffers, rec0 = p->gut_records, mask0 = p->fwd_masked_store, reg0 = p->reg_passes;
+  p->reg_passes = 0;
   double t[6] = {-1.0, -1.0, -1.0, -1.0, -1.0, -1.0};
   int best_buf = buf0, best_rec = rec0, best_mask = mask0;
   p->fwd_masked_store = p->gu_covered ? 1 : 0;
@@ -588,6 +609,17 @@ extern "C" int mlg_plan_autotune_variants(mlg_plan_t p, int reps, double* ms) {
     best_mask = t[5] < best_fwd ? 0 : 1;
   }
   p->fwd_masked_store = best_mask;
+  // the register passes (whole-grid stores never beat masked ones there)
+  // against the best of the above
+  int best_reg = reg0;
+  if (st == MLG_OK && best_fwd > 0.0) {
+    p->reg_passes = 1;
+    p->fwd_masked_store = p->gu_covered ? 1 : 0;
+    best_reg = time_it(true) < (t[5] > 0.0 ? std::min(best_fwd, t[5]) : best_fwd) ? 1 : 0;
+    if (best_reg) best_mask = p->fwd_masked_store;
+  }
+  p->reg_passes = best_reg;
+  p->fwd_masked_store = best_mask;
   if (st == MLG_OK && p->Gut_s.ord_rec && p->adjoint_mode == 2) {
     double best = 1e30;
     for (int v = 0; v <= 1 && st == MLG_OK; ++v) {
@@ -602,12 +634,14 @@ extern "C" int mlg_plan_autotune_variants(mlg_plan_t p, int reps, double* ms) {
   p->pass_buffers = buf0;
   p->gut_records = rec0;
   p->fwd_masked_store = mask0;
+  p->reg_passes = reg0;
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   if (ms)
     for (int i = 0; i < 6; ++i) ms[i] = t[i];
   if (st != MLG_OK) return st;
-  return mlg_plan_set_variant(p, best_buf, best_rec, best_mask);
+  MLG_TRY(mlg_plan_set_variant(p, best_buf, best_rec, best_mask));
+  return mlg_plan_set_register_passes(p, best_reg);
 }
 
 extern "C" int mlg_plan_set_precision(mlg_plan_t p, int precision) {

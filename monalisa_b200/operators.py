@@ -249,17 +249,25 @@ class NufftPlan:
         """The plan's kernel variants: {'pass_buffers': 0 (cp.async passes),
         2 or 3 (TMA passes with that many bundle buffers), 'gut_records': 0 (CSR
         rows) or 1 (row records), 'fwd_masked_store': 1 (the last forward pass
-        stores only the grid chunks holding cells Gu reads) or 0}."""
-        a, b, c = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+        stores only the grid chunks holding cells Gu reads) or 0,
+        'register_passes': 1 (the default: line passes through registers where
+        the axis length has them) or 0}.  Setting 'pass_buffers' without
+        'register_passes' selects those passes, i.e. 'register_passes': 0."""
+        a, b, c, r = ctypes.c_int(), ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         N.call("mlg_plan_get_variant", self._h, ctypes.byref(a), ctypes.byref(b), ctypes.byref(c))
-        return {"pass_buffers": a.value, "gut_records": b.value, "fwd_masked_store": c.value}
+        N.call("mlg_plan_get_register_passes", self._h, ctypes.byref(r))
+        return {"pass_buffers": a.value, "gut_records": b.value, "fwd_masked_store": c.value,
+                "register_passes": r.value}
 
     @variant.setter
     def variant(self, v: dict):
         cur = self.variant
+        if "pass_buffers" in v:
+            cur["register_passes"] = 0
         cur.update(v)
         N.call("mlg_plan_set_variant", self._h, int(cur["pass_buffers"]), int(cur["gut_records"]),
                int(cur["fwd_masked_store"]))
+        N.call("mlg_plan_set_register_passes", self._h, int(cur["register_passes"]))
 
     def status(self) -> None:
         """Synchronises the plan's stream; raises MonalisaError (timeout) when
