@@ -354,6 +354,9 @@ int mlg_idf(int imDim, const int* N_u, const float* dK_u, int nCol,
  * its occupancy bit is set (even nCh).  All give the same values up to
  * floating-point summation order of the long rows.  Tuning API; no reference
  * counterpart. */
+/* An odd coil count (2-D, 3-D; at most 32) with register passes
+ * (mlg_plan_set_register_passes) runs the masked strategy's kernels, a coil
+ * per thread, whichever strategy is set. */
 #define MLG_ADJ_FULL_GRID 0
 #define MLG_ADJ_FUSED 1
 #define MLG_ADJ_MASKED 2

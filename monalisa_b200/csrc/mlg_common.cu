@@ -93,6 +93,8 @@ void csr_free(Csr& c) {
   cudaFree(c.ord_bounds);
   cudaFree(c.val_h);
   cudaFree(c.ord_rec);
+  cudaFree(c.heavy_units);
+  cudaFree(c.heavy_multi);
   c = Csr();
 }
 
@@ -126,9 +128,9 @@ __global__ void nz_rows_kernel(const uint32_t* __restrict__ mask, const int* __r
 
 // brick key of row i (rows[i], or i): its cell (the row itself, or the
 // column of its first entry when by_first_col; empty rows sort last)
-// split: rows with more than kMidRow entries get the key's top bit (they
-// sort after the others, each group in brick order) and are counted in
-// n_mid.
+// split: the key is the brick and the row's entry count, in three groups: rows
+// of kFirstRow + 1 to kMidRow entries, shorter rows, and rows with more than
+// kMidRow entries (counted in n_mid), each group in brick order.
 __global__ void order_keys_kernel(const uint32_t* __restrict__ row_ptr, const int* __restrict__ col,
                                   const int* __restrict__ rows, int n, int by_first_col, int N0, int N1, int nbx,
                                   int nby, bool split, uint32_t* __restrict__ keys, int* __restrict__ vals,
@@ -148,9 +150,15 @@ __global__ void order_keys_kernel(const uint32_t* __restrict__ row_ptr, const in
     const long long x = cell % N0, t = cell / N0, y = t % N1, z = t / N1;
     const long long brick = (x >> 3) + nbx * ((y >> 3) + (long long)nby * (z >> 3));
     uint32_t key = (uint32_t)(brick * 512 + (x & 7) + 8 * ((y & 7) + 8 * (z & 7)));
-    if (split && row_ptr[r + 1] - row_ptr[r] > (uint32_t)kMidRow) {
-      key |= 0x80000000u;
-      atomicAdd(n_mid, 1);
+    if (split) {
+      const uint32_t n = row_ptr[r + 1] - row_ptr[r];
+      key = (uint32_t)brick * 128u + min(n, 127u);
+      if (n > (uint32_t)kMidRow) {
+        key |= 0x80000000u;
+        atomicAdd(n_mid, 1);
+      } else if (n <= (uint32_t)kFirstRow) {
+        key |= 0x40000000u;
+      }
     }
     keys[i] = key;
   }
@@ -162,6 +170,42 @@ __global__ void order_bounds_kernel(const uint32_t* __restrict__ row_ptr, const 
     const int r = rows[i];
     bounds[i] = make_uint2(row_ptr[r], row_ptr[r + 1]);
   }
+}
+
+// The heavy rows (ord_rows from ord_short on) cut into units of at most
+// kUnitLen entries, rows of several units first.
+static int csr_build_units(Csr& c, cudaStream_t s) {
+  const int nh = c.n_ord - c.ord_short;
+  if (nh <= 0) return MLG_OK;
+  std::vector<int> rows(nh);
+  std::vector<uint2> be(nh);
+  MLG_CUDA(cudaMemcpyAsync(rows.data(), c.ord_rows + c.ord_short, sizeof(int) * nh, cudaMemcpyDeviceToHost, s));
+  MLG_CUDA(cudaMemcpyAsync(be.data(), c.ord_bounds + c.ord_short, sizeof(uint2) * nh, cudaMemcpyDeviceToHost, s));
+  MLG_CUDA(cudaStreamSynchronize(s));
+  std::vector<int4> units, single;
+  std::vector<int2> multi;
+  for (int i = 0; i < nh; ++i) {
+    const uint32_t b = be[i].x, n = be[i].y - be[i].x;
+    if (n <= (uint32_t)kUnitLen) {
+      single.push_back(make_int4(rows[i], (int)b, (int)be[i].y, -1));
+      continue;
+    }
+    const int k = (int)((n + kUnitLen - 1) / kUnitLen);
+    for (int j = 0; j < k; ++j)  // units of about equal length
+      units.push_back(make_int4(rows[i], (int)(b + (uint32_t)((unsigned long long)n * j / k)),
+                                (int)(b + (uint32_t)((unsigned long long)n * (j + 1) / k)), (int)multi.size()));
+    multi.push_back(make_int2((int)units.size() - k, k));
+  }
+  c.n_multi = (int)multi.size();
+  c.n_multi_units = (int)units.size();
+  units.insert(units.end(), single.begin(), single.end());
+  c.n_units = (int)units.size();
+  MLG_CUDA(cudaMalloc(&c.heavy_units, sizeof(int4) * units.size()));
+  MLG_CUDA(cudaMalloc(&c.heavy_multi, sizeof(int2) * std::max<size_t>(1, multi.size())));
+  MLG_CUDA(cudaMemcpyAsync(c.heavy_units, units.data(), sizeof(int4) * units.size(), cudaMemcpyHostToDevice, s));
+  MLG_CUDA(cudaMemcpyAsync(c.heavy_multi, multi.data(), sizeof(int2) * multi.size(), cudaMemcpyHostToDevice, s));
+  MLG_CUDA(cudaStreamSynchronize(s));
+  return MLG_OK;
 }
 
 int csr_build_order(Csr& c, const int* N, bool nonempty, cudaStream_t s) {
@@ -214,7 +258,7 @@ int csr_build_order(Csr& c, const int* N, bool nonempty, cudaStream_t s) {
   c.n_ord = n;
   c.ord_nonempty = nonempty;
   c.ord_short = split ? n - h_mid : -1;
-  return MLG_OK;
+  return split ? csr_build_units(c, s) : MLG_OK;
 }
 
 int csr_build_nonempty(Csr& c, cudaStream_t s) {

@@ -118,11 +118,15 @@ struct DevBuf {
 // jump format squeezes out are empty).  Long rows (more than kLongRow
 // entries) are listed separately so that one CTA can split them.
 constexpr int kLongRow = 256;
-// rows with more than kMidRow (and at most kLongRow) entries are gathered by
-// a warp each inside the operators (measured on Gut: 16, 32, 64, 128 entries
-// gave 0.797 / 0.769 / 0.757 / 0.749 ms on the 4096-spoke 16-coil koosh
-// case and 0.243 / 0.233 / 0.228 / 0.266 ms on a 1500-spoke 12-coil one)
+// rows with more than kMidRow entries are gathered inside the operators as
+// units of at most kUnitLen entries, a CTA each (heavy_unit)
 constexpr int kMidRow = 64;
+constexpr int kUnitLen = 256;
+// short rows with more than kFirstRow entries (the neighbourhood of the k-space
+// centre) are gathered first: a block of them runs several times as long as
+// the others and would be the product's tail (192^3 x 12 coils: 113 -> 98 us;
+// 8, 16 and 32 measured alike)
+constexpr int kFirstRow = 16;
 
 struct Csr {
   int r_size = 0;         // number of columns
@@ -155,8 +159,16 @@ struct Csr {
   int n_ord = 0;
   bool ord_nonempty = false;
   // non-empty order only: the first ord_short rows have at most kMidRow
-  // entries, the rest more (each part in block order); -1: not split
+  // entries -- those with more than kFirstRow first -- the rest more (each
+  // part in block order, the short rows of a block by entry count); -1: not
+  // split
   int ord_short = -1;
+  // units of the rows with more than kMidRow entries: (row, first entry, end,
+  // m): m >= 0: one of several units of heavy_multi[m] = (first unit, units),
+  // which come first (n_multi_units of them); -1: the whole row
+  int4* heavy_units = nullptr;
+  int2* heavy_multi = nullptr;
+  int n_units = 0, n_multi = 0, n_multi_units = 0;
   // FP16 copy of val for the mixed-precision solver (built on demand)
   __half* val_h = nullptr;
   // Row records of the first ord_short ordered rows (sign-folded copies
@@ -194,9 +206,11 @@ int csr_build_segments(Csr& c, cudaStream_t s);
 // Builds nz_rows / nz_mask (idempotent).
 int csr_build_nonempty(Csr& c, cudaStream_t s);
 // Builds ord_rows / ord_bounds (idempotent): the non-empty rows (nonempty;
-// rows are cells of the grid N) or all rows (rows keyed by the cell of their
-// first entry; empty rows last), in order of 8 x 8 x 8 bricks of cells, x
-// fastest within a brick; ties keep row order.  Needs nz_rows for nonempty.
+// rows are cells of the grid N; the heavy units with them) or all rows (rows
+// keyed by the cell of their first entry; empty rows last), in order of
+// 8 x 8 x 8 bricks of cells -- the non-empty ones by entry count within a
+// brick, so that the rows a warp gathers together have equal counts -- ties
+// in row order.  Needs nz_rows for nonempty.
 int csr_build_order(Csr& c, const int* N, bool nonempty, cudaStream_t s);
 
 }  // namespace mlg
@@ -277,6 +291,10 @@ struct SpmmArgs {
   // records (ord_rec), when built (FP32 values, rounded to FP16 as read with
   // half_values)
   bool records = false;
+  // Counters of the heavy rows of several units (>= m->n_multi, zero between
+  // products; one set per stream of products).  NULL: the ordered product
+  // takes the segment kernels for its long rows instead.
+  unsigned* unit_count = nullptr;
   // Optional: raised (atomicMax on the bits) to the largest |re| or |im| of
   // the values written, before any FP16 rounding (device, non-negative float)
   unsigned* absmax = nullptr;

@@ -46,6 +46,7 @@ static void box_strides(const int e[3], int C, long long st[3]) {
 // cells Gu reads (plan variant fwd_masked_store; the line masks of the
 // masked adjoint cover every Gu column when gu_covered).
 static void set_masked_store(const mlg_plan_s* p, PassDesc& pd) {
+  if (p->odd_masked && p->odd_covered && p->reg_passes) pd.out_tmask = p->tmask;
   if (p->fwd_masked_store && p->gu_covered && p->line_mask) {
     pd.out_lmask = p->line_mask;
     pd.out_tmask = p->tmask;
@@ -136,7 +137,10 @@ static int forward_pass(mlg_plan_s* p, int ax, const float2* x, bool x_per_coil,
 // reads the grid written by the Gut product.
 enum : int { kAdjFullGrid = 0, kAdjFused = 1, kAdjMasked = 2 };
 
-static bool fused_gut(const mlg_plan_s* p) { return p->adjoint_mode == kAdjFused; }
+// the strategy an adjoint runs (see odd_masked)
+static int run_mode(const mlg_plan_s* p) { return p->odd_masked && p->reg_passes ? (int)kAdjMasked : p->adjoint_mode; }
+
+static bool fused_gut(const mlg_plan_s* p) { return run_mode(p) == kAdjFused; }
 
 // adjoint variants a plan can run
 bool adjoint_mode_valid(const mlg_plan_s* p, int mode) {
@@ -187,7 +191,7 @@ static int inverse_pass(mlg_plan_s* p, int ax, const float2* y, const float* HY,
   }
   const bool gut_in = fused_gut(p) && ax == d - 1;
   if (gut_in) set_gut_input(p, pd, y, HY);
-  if (p->adjoint_mode == kAdjMasked && ax == d - 1) {
+  if (run_mode(p) == kAdjMasked && ax == d - 1) {
     pd.in_mask = p->Gut_s.nz_mask;
     pd.in_lmask = p->line_mask;
     pd.tmask = p->tmask;
@@ -323,8 +327,9 @@ int nakatsha_stage(mlg_plan_s* p, int stage, const float2* y, const float* HY, f
     a.out.a = p->grid;
     a.out.rows = p->Nu_tot;
     a.long_only = fused_gut(p);
-    a.nonempty_only = p->adjoint_mode == kAdjMasked;
+    a.nonempty_only = run_mode(p) == kAdjMasked;
     a.records = p->gut_records != 0;
+    a.unit_count = p->unit_count;
     a.seg_scratch = p->seg_scratch;
     if (half_b(p)) {
       MLG_CUDA(cudaMemsetAsync(p->mix_amax + 1, 0, sizeof(unsigned), s));
@@ -473,7 +478,7 @@ __global__ void cover_check_kernel(const int* __restrict__ col, long long nnz, c
 // Whether the line masks cover every cell Gu reads (Gu and Gut of one
 // trajectory are transposes, so they do; matrices from elsewhere may not).
 static int check_gu_covered(mlg_plan_s* p, cudaStream_t s) {
-  p->gu_covered = false;
+  p->gu_covered = p->odd_covered = false;
   if (!p->line_mask || !p->Gu || !p->Gut_s.nz_mask || p->Gu_s.nnz == 0) return MLG_OK;
   DevBuf<int> miss;
   MLG_TRY(miss.alloc(1, s));
@@ -483,7 +488,7 @@ static int check_gu_covered(mlg_plan_s* p, cudaStream_t s) {
   int h = 1;
   MLG_CUDA(cudaMemcpyAsync(&h, miss.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   MLG_CUDA(cudaStreamSynchronize(s));
-  p->gu_covered = h == 0;
+  (p->nCh % 2 ? p->odd_covered : p->gu_covered) = h == 0;
   return MLG_OK;
 }
 
@@ -641,15 +646,17 @@ static int plan_create_impl(int imDim, const int* N_u, const int* n_u, int nCh, 
   // nearby cells) live with the caller's matrix (built once, shared by the
   // sign-folded copy)
   if (Gu && (st = csr_sign_copy(*Gu, false, imDim, p->N, sc, p->Gu_s, s)) != MLG_OK) return bail(st);
-  if (Gut && (nCh % 2) == 0 && (st = csr_build_nonempty(const_cast<Csr&>(*Gut), s)) != MLG_OK) return bail(st);
-  if (Gut && (nCh % 2) == 0 && (st = csr_build_order(const_cast<Csr&>(*Gut), p->N, true, s)) != MLG_OK)
-    return bail(st);
+  const bool odd = (nCh % 2) == 1 && nCh <= 32 && imDim >= 2 && p->ax[imDim - 1].rA > 0;
+  const bool tables = Gut && ((nCh % 2) == 0 || odd);
+  if (tables && (st = csr_build_nonempty(const_cast<Csr&>(*Gut), s)) != MLG_OK) return bail(st);
+  if (tables && (st = csr_build_order(const_cast<Csr&>(*Gut), p->N, true, s)) != MLG_OK) return bail(st);
   if (Gut && (st = csr_sign_copy(*Gut, true, imDim, p->N, 1.0f, p->Gut_s, s)) != MLG_OK) return bail(st);
-  if (Gut && (nCh % 2) == 0 && nCh / 2 <= 16 && (st = csr_build_records(p->Gut_s, s)) != MLG_OK) return bail(st);
+  if (tables && nCh / 2 <= 16 && (st = csr_build_records(p->Gut_s, s)) != MLG_OK) return bail(st);
   p->reg_passes = register_passes_default() ? 1 : 0;
-  p->gut_records = p->Gut_s.ord_rec ? 1 : 0;  // measured faster on c2 (0.607 vs 0.671 ms)
-  if ((st = build_line_mask(p, s)) != MLG_OK) return bail(st);
+  p->gut_records = p->Gut_s.ord_rec && !odd ? 1 : 0;  // measured faster on c2 (0.607 vs 0.671 ms)
+  if (tables && (st = build_line_mask(p, s)) != MLG_OK) return bail(st);
   if ((st = check_gu_covered(p, s)) != MLG_OK) return bail(st);
+  p->odd_masked = odd && p->Gut_s.ord_rec && p->Gut_s.ord_short >= 0 && p->tmask;
   p->fwd_masked_store = p->gu_covered ? 1 : 0;
   p->adjoint_mode = adjoint_mode_valid(p, kAdjMasked) ? kAdjMasked : (imDim >= 2 ? kAdjFused : kAdjFullGrid);
   const size_t kbytes = sizeof(float2) * (size_t)nu * nCh;
@@ -690,12 +697,15 @@ static int plan_create_impl(int imDim, const int* N_u, const int* n_u, int nCh, 
   p->partial_cap = cap;
   const size_t seg_floats = std::max<size_t>(
       1, std::max(Gu ? spmm_scratch_floats(*Gu, nCh) : 0, Gut ? spmm_scratch_floats(*Gut, nCh) : 0));
+  const size_t n_multi = Gut ? std::max(1, Gut->n_multi) : 1;
   if (cudaMalloc(&p->partial, sizeof(double) * (size_t)cap) != cudaSuccess ||
-      cudaMalloc(&p->seg_scratch, sizeof(float) * seg_floats) != cudaSuccess ||
+      cudaMalloc(&p->seg_scratch, sizeof(float) * (seg_floats + n_multi)) != cudaSuccess ||
+      cudaMemsetAsync(p->seg_scratch + seg_floats, 0, sizeof(float) * n_multi, s) != cudaSuccess ||
       cudaMalloc(&p->scalars, sizeof(double) * 64) != cudaSuccess) {
     cudaGetLastError();
     return bail(fail(MLG_ERR_OOM, "plan: partial buffer allocation failed"));
   }
+  p->unit_count = reinterpret_cast<unsigned*>(p->seg_scratch + seg_floats);
   if (cudaStreamSynchronize(s) != cudaSuccess) return bail(fail(MLG_ERR_CUDA, "plan creation failed"));
   p->bytes = (share ? 0 : 2 * kbytes + gbytes + abytes + bbytes) +
              sizeof(float) * (size_t)((Gu ? Gu->nnz : 0) + (Gut ? Gut->nnz : 0)) + sizeof(double) * (cap + 64) +

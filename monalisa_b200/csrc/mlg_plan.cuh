@@ -29,7 +29,8 @@ struct mlg_plan_s {
   mlg::FftAxisPlan ax[3];
   double* partial = nullptr;      // FP64 partial sums (CTA results)
   int partial_cap = 0;
-  float* seg_scratch = nullptr;   // long-row segment partials of Gu / Gut
+  float* seg_scratch = nullptr;   // long-row segment / heavy-unit partials of Gu / Gut
+  unsigned* unit_count = nullptr; // SpmmArgs::unit_count of Gut's products (in seg_scratch's allocation)
   // How the adjoint feeds its first inverse pass:
   //  0 kAdjFullGrid: Gut writes every grid cell, the pass streams the grid;
   //  1 kAdjFused:    the pass gathers Gut rows from k-space itself (2-D/3-D);
@@ -39,6 +40,11 @@ struct mlg_plan_s {
   // Gut's occupancy bits regrouped per line of the first inverse pass (axis
   // imDim - 1): line_mask_words words per line (built with the occupancy
   // tables, for kAdjMasked)
+  // Odd coil counts (2-D, 3-D) with register passes: whatever the strategy
+  // set, the adjoint runs as kAdjMasked does for even ones -- Gut's non-empty
+  // rows a coil per thread, occupancy bits in the first pass -- and the last
+  // forward pass stores masked where Gu's columns are covered (odd_covered)
+  bool odd_masked = false, odd_covered = false;
   uint32_t* line_mask = nullptr;
   int line_mask_words = 0;
   // the same bits regrouped for the register passes (PassDesc::tmask; in

@@ -507,7 +507,7 @@ extern "C" int mlg_plan_set_variant(mlg_plan_t p, int pass_buffers, int gut_reco
   MLG_CHECK((pass_buffers == 0 || pass_buffers == 2 || pass_buffers == 3) && (gut_records == 0 || gut_records == 1) &&
                 (fwd_masked_store == 0 || fwd_masked_store == 1),
             "variants: pass_buffers 0, 2 or 3; gut_records 0 or 1; fwd_masked_store 0 or 1");
-  MLG_CHECK(!gut_records || p->Gut_s.ord_rec, "this plan has no Gut row records (masked adjoint, even coil count)");
+  MLG_CHECK(!gut_records || (p->Gut_s.ord_rec && p->nCh % 2 == 0), "this plan has no Gut row records (masked adjoint, even coil count)");
   MLG_CHECK(!fwd_masked_store || p->gu_covered,
             "this plan cannot mask its forward stores (no line masks, or a Gu column outside Gut's occupied cells)");
   if (p->reg_passes || p->pass_buffers != pass_buffers || p->gut_records != gut_records ||

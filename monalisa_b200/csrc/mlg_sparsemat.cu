@@ -43,7 +43,7 @@ struct SpmmParams {
   double* partial;
   int partial_long_offset;
   unsigned* absmax;
-  // FP16 point-layout input (pair kernel, IN_H): scale from this word and length
+  // FP16 point-layout input (spmm_fwd_kernel, IN_H): scale from this word and length
   const unsigned* in_h_amax;
   int in_h_len;
 };
@@ -254,123 +254,169 @@ __global__ void __launch_bounds__(256) spmm_seg_combine_kernel(SpmmParams p, con
   }
 }
 
-// Point layout in and out, even nCh: a thread owns a (row, coil pair) output
-// and moves 16 bytes per load/store; the row's column/value stream is read
-// once per pair instead of once per coil.  `rows` (optional) lists the rows
-// to compute, in that order (the matrix's ord_rows: non-empty rows, or all
-// rows, in blocks of nearby cells), and `bounds` their entry ranges; other
-// rows are left untouched.  Entries
-// are summed in stored order with round-to-nearest multiply/add, or, with
-// CONTRACT (operators inside plans), with the row scale folded into the
-// matrix value and fused multiply-adds: 9 instead of 16 arithmetic and load
-// instructions per entry and coil pair.
-// A coil pair: two complex values (float4) in and out.
-
-struct MidRows {
-  const int* rows = nullptr;
-  const uint2* bounds = nullptr;
-  int n = 0;
-  int blocks = 0;
+// Rows with more than kMidRow entries inside the operators, cut into units of
+// at most kUnitLen entries (Csr::heavy_units).
+struct HeavyUnits {
+  const int4* units = nullptr;
+  const int2* multi = nullptr;
+  int n = 0;                  // units = first blocks of the launch
+  float* scratch = nullptr;   // partial sums of the multi-unit rows' units
+  unsigned* count = nullptr;  // finished units per multi-unit row
 };
 
-// Rows with kMidRow < n <= kLongRow entries inside the operators (CONTRACT
-// semantics, FP32 point layout in and out, no partials): a warp per row at
-// a time, lane = (entry group eg, coil pair pi) for P <= 16 pairs, EG = 32 /
-// P groups; group eg takes entries eg, eg + EG, ... and the groups' sums are
-// added in group order (a fixed order: deterministic, but not the row's
-// stored order).  AM: p.absmax is raised to the largest output component.
-template <bool AM>
-__device__ __forceinline__ void mid_rows_block(const SpmmParams& p, const int* __restrict__ rows,
-                                               const uint2* __restrict__ bounds, int n_rows, int block,
-                                               int nblocks) {
-  const int P = p.nCh >> 1, EG = 32 / P;
-  const int lane = threadIdx.x & 31, eg = lane / P, pi = lane - eg * P;
-  const bool active = eg < EG;
+__device__ __forceinline__ void fma_to(float4& a, float m, float4 v) {
+  const float2 lo = __ffma2_rn(make_float2(m, m), make_float2(v.x, v.y), make_float2(a.x, a.y));
+  const float2 hi = __ffma2_rn(make_float2(m, m), make_float2(v.z, v.w), make_float2(a.z, a.w));
+  a = make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ void fma_to(float2& a, float m, float2 v) { a = __ffma2_rn(make_float2(m, m), v, a); }
+__device__ __forceinline__ float4 add_to(float4 a, float4 b) {
+  return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+__device__ __forceinline__ float2 add_to(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float4 scaled(float4 a, float f) {
+  return make_float4(__fmul_rn(a.x, f), __fmul_rn(a.y, f), __fmul_rn(a.z, f), __fmul_rn(a.w, f));
+}
+__device__ __forceinline__ float2 scaled(float2 a, float f) { return make_float2(__fmul_rn(a.x, f), __fmul_rn(a.y, f)); }
+__device__ __forceinline__ float abs_max4(float2 v) { return fmaxf(fabsf(v.x), fabsf(v.y)); }
+__device__ __forceinline__ double sqnorm(float4 a) {
+  return (double)a.x * a.x + (double)a.y * a.y + (double)a.z * a.z + (double)a.w * a.w;
+}
+__device__ __forceinline__ double sqnorm(float2 a) { return (double)a.x * a.x + (double)a.y * a.y; }
+template <class VT>
+__device__ __forceinline__ VT vzero();
+template <>
+__device__ __forceinline__ float4 vzero<float4>() { return make_float4(0.f, 0.f, 0.f, 0.f); }
+template <>
+__device__ __forceinline__ float2 vzero<float2>() { return make_float2(0.f, 0.f); }
+
+// One heavy unit by one CTA of 256 threads (operator semantics: the row scale
+// folded into the matrix value, fused multiply-adds, FP32 point layout; VT =
+// float4: a coil pair per thread, float2: a coil): thread = (entry group eg,
+// coil column pi), group eg takes entries eg, eg + EG, ... four at a time in
+// flight, the groups' sums are added in a fixed tree.  A unit that is a whole
+// row stores it; the units of a longer row leave their sums in scratch and
+// the last one to finish adds them in a fixed order (deterministic).
+//
+// A warp per such row left a chain of up to 52 dependent gathers (60 us in
+// 2-D, where nothing covers it), and the rows above 256 entries took two more
+// launches (33 of 135 us on an eighth of the 4096-spoke case).
+template <class VT, bool AM>
+__device__ __forceinline__ void heavy_unit(const SpmmParams& p, const HeavyUnits& H, int unit) {
+  __shared__ VT red[256];
+  __shared__ bool last;
+  const int P = p.nCh / (int)(sizeof(VT) / sizeof(float2)), EG = 256 / P;
+  const int eg = threadIdx.x / P, pi = threadIdx.x - eg * P;
   const bool scale = p.in_row_scale != nullptr;
-  const float4* in = reinterpret_cast<const float4*>(p.in.a);
-  float amax = 0.f;
-  for (int i = block * 8 + (int)(threadIdx.x >> 5); i < n_rows; i += nblocks * 8) {
-    const uint2 be = __ldg(bounds + i);
-    if (be.y - be.x > (uint32_t)kLongRow) continue;  // segment kernels own it (uniform in the warp)
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (active) {
-      for (uint32_t k = be.x + eg; k < be.y; k += EG) {
-        const int j = __ldg(p.col + k);
-        float m = val_at(p, k);
-        if (scale) m = __fmul_rn(m, __ldg(p.in_row_scale + j));
-        const float4 v = __ldg(in + (long long)j * P + pi);
-        acc.x = __fmaf_rn(m, v.x, acc.x);
-        acc.y = __fmaf_rn(m, v.y, acc.y);
-        acc.z = __fmaf_rn(m, v.z, acc.z);
-        acc.w = __fmaf_rn(m, v.w, acc.w);
+  const VT* in = reinterpret_cast<const VT*>(p.in.a);
+  const int4 u = __ldg(H.units + unit);
+  VT acc = vzero<VT>();
+  if (eg < EG) {
+    for (uint32_t k = (uint32_t)u.y + eg; k < (uint32_t)u.z; k += 4 * EG) {
+      int j[4];
+      float m[4];
+      VT v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t kq = k + q * EG;
+        const bool ok = kq < (uint32_t)u.z;
+        j[q] = ok ? __ldg(p.col + kq) : -1;
+        m[q] = ok ? val_at(p, kq) : 0.f;
       }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        v[q] = vzero<VT>();
+        if (j[q] >= 0) {
+          v[q] = __ldg(in + (long long)j[q] * P + pi);
+          if (scale) m[q] = __fmul_rn(m[q], __ldg(p.in_row_scale + j[q]));
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) fma_to(acc, m[q], v[q]);  // (past the end: 0 * 0)
     }
-    float4 s = acc;
-    for (int e = 1; e < EG; ++e) {  // lanes of group 0 add the other groups in order
-      const int src = pi + e * P;
-      s.x += __shfl_sync(0xffffffffu, acc.x, src);
-      s.y += __shfl_sync(0xffffffffu, acc.y, src);
-      s.z += __shfl_sync(0xffffffffu, acc.z, src);
-      s.w += __shfl_sync(0xffffffffu, acc.w, src);
+  }
+  int top = 1;
+  while (top < EG) top <<= 1;
+  auto tree = [&](VT x) {  // the sum over the entry groups, in group 0
+    red[threadIdx.x] = x;
+    for (int w = top >> 1; w > 0; w >>= 1) {
+      __syncthreads();
+      if (eg < w && eg + w < EG) red[threadIdx.x] = add_to(red[threadIdx.x], red[threadIdx.x + w * P]);
     }
+    __syncthreads();
+    return red[threadIdx.x];
+  };
+  acc = tree(acc);
+  bool store = eg == 0;
+  if (u.w >= 0) {
+    VT* part = reinterpret_cast<VT*>(H.scratch);
+    const int2 mu = __ldg(H.multi + u.w);
     if (eg == 0) {
-      if (p.out_scale != 1.0f)
-        s = make_float4(__fmul_rn(s.x, p.out_scale), __fmul_rn(s.y, p.out_scale), __fmul_rn(s.z, p.out_scale),
-                        __fmul_rn(s.w, p.out_scale));
-      reinterpret_cast<float4*>(p.out.a)[(long long)__ldg(rows + i) * P + pi] = s;
-      if constexpr (AM) amax = fmaxf(amax, abs_max4(s));
+      part[(long long)unit * P + pi] = acc;
+      __threadfence();
     }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      last = atomicAdd(H.count + u.w, 1u) == (unsigned)(mu.y - 1);
+      if (last) H.count[u.w] = 0u;
+      __threadfence();
+    }
+    __syncthreads();
+    if (last) {
+      VT sum = vzero<VT>();
+      if (eg < EG)
+        for (int k = eg; k < mu.y; k += EG) sum = add_to(sum, __ldcg(part + (long long)(mu.x + k) * P + pi));
+      acc = tree(sum);
+    } else {
+      store = false;
+    }
+  }
+  float amax = 0.f;
+  if (store) {
+    if (p.out_scale != 1.0f) acc = scaled(acc, p.out_scale);
+    reinterpret_cast<VT*>(p.out.a)[(long long)u.x * P + pi] = acc;
+    amax = abs_max4(acc);
   }
   if constexpr (AM) block_absmax(p.absmax, amax);  // every thread of the block reaches it
 }
 
-// PPT coil pairs per thread: the row's bounds and each entry's column and
-// value are loaded once for PPT pairs.  Per coil the entries are summed in
-// the same order for every PPT, so the outputs do not depend on it.
-// Resident blocks per SM: the gathers are latency-bound, so occupancy beats
-// spill-free code -- one pair per thread at 8 blocks (32 registers, a few
-// spilled bytes) took Gut on the 4096-spoke 16-coil koosh case from 0.757
-// (6 blocks) to 0.671 ms; 5 blocks gave 0.841 ms.
-template <int PPT>
-constexpr int pair_min_blocks() {
-  return PPT == 1 ? 8 : (PPT == 2 ? 5 : 4);
-}
-
-// With mid_blocks > 0 (CONTRACT, FP32 output) the first mid_blocks blocks
-// gather the mid rows, a warp per row (mid_rows_block), and the others the
-// listed short rows: one launch, the long-running mid rows started first.
-// IN_H: the input holds __half2 values times a power of two (the
-// mixed-precision forward grid; the scale as its writer computed it from
-// p.in_h_amax / p.in_h_len), read as 8 bytes per coil pair.
-template <bool CONTRACT, int PPT, bool IN_H = false>
-__global__ void __launch_bounds__(256, pair_min_blocks<PPT>()) spmm_pair_kernel(SpmmParams p,
-                                                                               const int* __restrict__ rows,
-                                                                               const uint2* __restrict__ bounds,
-                                                                               int n_rows, MidRows mid) {
-  __shared__ double sh[32];
-  if ((int)blockIdx.x < mid.blocks) {
-    if constexpr (CONTRACT) {
+// Operator products whose input rows are scaled (the adjoint without row
+// records, or of every row), point layout in and out, even nCh: a thread owns
+// a (row, coil pair) output and moves 16 bytes per load and store; the row's
+// column/value stream is read once per pair instead of once per coil.  `rows`
+// (optional) lists the rows to compute, in that order (the matrix's ord_rows),
+// and `bounds` their entry ranges; other rows are left untouched.  Entries are
+// summed in stored order with the row scale folded into the matrix value and
+// fused multiply-adds.  Eight 256-thread blocks per SM (32 registers, a few
+// spilled bytes): the gathers are latency-bound.  HEAVY: the first heavy.n
+// blocks gather the heavy units, a CTA each (heavy_unit), the others the
+// listed short rows: one launch, the longest-running blocks first.
+template <bool HEAVY>
+__global__ void __launch_bounds__(256, 8) spmm_pair_kernel(SpmmParams p, const int* __restrict__ rows,
+                                                           const uint2* __restrict__ bounds, int n_rows,
+                                                           HeavyUnits heavy) {
+  int bid = (int)blockIdx.x;
+  if constexpr (HEAVY) {
+    if (bid < heavy.n) {
       if (p.absmax)
-        mid_rows_block<true>(p, mid.rows, mid.bounds, mid.n, blockIdx.x, mid.blocks);
+        heavy_unit<float4, true>(p, heavy, bid);
       else
-        mid_rows_block<false>(p, mid.rows, mid.bounds, mid.n, blockIdx.x, mid.blocks);
+        heavy_unit<float4, false>(p, heavy, bid);
+      return;
     }
-    return;
+    bid -= heavy.n;
   }
-  const int bid = (int)blockIdx.x - mid.blocks;
-  const int P = p.nCh >> 1, G = P / PPT;  // pairs per row, thread groups per row
+  const int P = p.nCh >> 1;
   const long long i0 = (long long)bid * p.rows_per_block;
   const int nr = (int)min((long long)p.rows_per_block, (long long)n_rows - i0);
-  const int total = nr * G;
+  const int total = nr * P;
   const bool scale = p.in_row_scale != nullptr;
-  const float hin = IN_H ? 1.f / half_store_scale(p.in_h_amax, p.in_h_len) : 1.f;  // a power of two
+  const float4* in = reinterpret_cast<const float4*>(p.in.a);
   float amax = 0.f;
-  double sq = 0.0;
-  // item -> row, first coil pair and entry range (empty for rows the segment kernels own)
-  auto fetch = [&](int it, long long& r, int& pi, uint32_t& b, uint32_t& n) {
-    const int lr = it / G;
-    pi = (it - lr * G) * PPT;
-    uint32_t e;
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    const int lr = it / P, pi = it - lr * P;
+    long long r;
+    uint32_t b, e;
     if (rows) {  // listed rows: bounds loaded beside the row index, not after it
       r = __ldg(rows + i0 + lr);
       const uint2 be = __ldg(bounds + i0 + lr);
@@ -381,142 +427,163 @@ __global__ void __launch_bounds__(256, pair_min_blocks<PPT>()) spmm_pair_kernel(
       b = __ldg(p.row_ptr + r);
       e = __ldg(p.row_ptr + r + 1);
     }
-    n = e - b;
-  };
-  auto entry = [&](uint32_t k, int pi, float4* acc) {
-    const int j = __ldg(p.col + k);
-    float m = val_at(p, k);
-    float4 v[PPT];
-    if constexpr (IN_H) {
-      const uint2* src = reinterpret_cast<const uint2*>(p.in.a) + (long long)j * P + pi;
-#pragma unroll
-      for (int u = 0; u < PPT; ++u) {
-        const uint2 q = __ldg(src + u);
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
-        const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
-        v[u] = make_float4(a.x * hin, a.y * hin, b.x * hin, b.y * hin);
-      }
-    } else {
-      const float4* src = reinterpret_cast<const float4*>(p.in.a) + (long long)j * P + pi;
-#pragma unroll
-      for (int u = 0; u < PPT; ++u) v[u] = __ldg(src + u);
-    }
-    if constexpr (CONTRACT) {
+    if (e - b > (uint32_t)kLongRow) continue;  // segment kernels own it
+    float4 acc = vzero<float4>();
+#pragma unroll 4
+    for (uint32_t k = b; k < e; ++k) {
+      const int j = __ldg(p.col + k);
+      float m = val_at(p, k);
+      const float4 v = __ldg(in + (long long)j * P + pi);
       if (scale) m = __fmul_rn(m, __ldg(p.in_row_scale + j));
-#pragma unroll
-      for (int u = 0; u < PPT; ++u) {
-        acc[u].x = __fmaf_rn(m, v[u].x, acc[u].x);
-        acc[u].y = __fmaf_rn(m, v[u].y, acc[u].y);
-        acc[u].z = __fmaf_rn(m, v[u].z, acc[u].z);
-        acc[u].w = __fmaf_rn(m, v[u].w, acc[u].w);
-      }
-    } else {
-      const float h = scale ? __ldg(p.in_row_scale + j) : 1.f;
-#pragma unroll
-      for (int u = 0; u < PPT; ++u) {
-        float4 w = v[u];
-        if (scale) w = make_float4(__fmul_rn(h, w.x), __fmul_rn(h, w.y), __fmul_rn(h, w.z), __fmul_rn(h, w.w));
-        acc[u].x = __fadd_rn(acc[u].x, __fmul_rn(m, w.x));
-        acc[u].y = __fadd_rn(acc[u].y, __fmul_rn(m, w.y));
-        acc[u].z = __fadd_rn(acc[u].z, __fmul_rn(m, w.z));
-        acc[u].w = __fadd_rn(acc[u].w, __fmul_rn(m, w.w));
-      }
+      fma_to(acc, m, v);
     }
-  };
-  auto finish_pair = [&](long long r, int pi, float4 acc, double w) {
-    if (p.out_scale != 1.0f)
-      acc = make_float4(__fmul_rn(acc.x, p.out_scale), __fmul_rn(acc.y, p.out_scale), __fmul_rn(acc.z, p.out_scale),
-                        __fmul_rn(acc.w, p.out_scale));
+    if (p.out_scale != 1.0f) acc = scaled(acc, p.out_scale);
     reinterpret_cast<float4*>(p.out.a)[r * P + pi] = acc;
     amax = fmaxf(amax, abs_max4(acc));
-    if (p.partial)
-      sq += w * ((double)acc.x * acc.x + (double)acc.y * acc.y + (double)acc.z * acc.z + (double)acc.w * acc.w);
-  };
-  for (int it = threadIdx.x; it < total; it += blockDim.x) {
-    long long r;
-    int pi;
-    uint32_t b, n;
-    fetch(it, r, pi, b, n);
-    if (n > (uint32_t)kLongRow) continue;  // segment kernels own it
-    float4 acc[PPT];
-#pragma unroll
-    for (int u = 0; u < PPT; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-    for (uint32_t k = b; k < b + n; ++k) entry(k, pi, acc);
-    const double w = p.partial && p.sqn_w ? (double)__ldg(p.sqn_w + r) : 1.0;
-#pragma unroll
-    for (int u = 0; u < PPT; ++u) finish_pair(r, pi + u, acc[u], w);
   }
   if (p.absmax) block_absmax(p.absmax, amax);
+}
+
+// VT values at an index of the input: FP32, or (IN_H) __half2 values times a
+// power of two (the mixed-precision forward grid), 8 bytes per coil pair.
+template <class VT, bool IN_H>
+struct GridIn {
+  using T = VT;
+  static __device__ __forceinline__ VT at(const T* a, float) { return __ldg(a); }
+};
+template <>
+struct GridIn<float4, true> {
+  using T = uint2;
+  static __device__ __forceinline__ float4 at(const T* a, float hin) {
+    const uint2 q = __ldg(a);
+    const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
+    const float2 y = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
+    return make_float4(x.x * hin, x.y * hin, y.x * hin, y.y * hin);
+  }
+};
+
+__device__ __forceinline__ float4 mul_add_rn(float4 a, float m, float4 v) {
+  return make_float4(__fadd_rn(a.x, __fmul_rn(m, v.x)), __fadd_rn(a.y, __fmul_rn(m, v.y)),
+                     __fadd_rn(a.z, __fmul_rn(m, v.z)), __fadd_rn(a.w, __fmul_rn(m, v.w)));
+}
+__device__ __forceinline__ float2 mul_add_rn(float2 a, float m, float2 v) {
+  return make_float2(__fadd_rn(a.x, __fmul_rn(m, v.x)), __fadd_rn(a.y, __fmul_rn(m, v.y)));
+}
+
+// Products of all rows without scales, point layout: the forward operator
+// (CONTRACT: fused multiply-adds) and the plain complex product (separate
+// round-to-nearest multiply and add: bit-identical to the reference's CPU
+// products), entries in stored order; a thread per (row, coil pair; VT =
+// float2: coil).  Latency-bound gathers of rows of equal length (27 entries in
+// 3-D): the columns, gathers and values of kFwdBatch entries are issued as
+// three groups before any is used.  Left to the compiler (unroll 4 at eight
+// blocks per SM, 32 registers) the loads of a batch waited for each other; at
+// six blocks (40 registers) four entries in flight take the 256^3 x 16-coil
+// product from 414 to 308 us, 192^3 x 12 coils 105 -> 75, 160 x 160 x 120 x 8
+// coils 62 -> 45, 512^2 x 12 coils 24 -> 19 us (3 entries at 6 blocks 316,
+// 5 at 5 blocks 314, 6 at 5 339, 4 at 8 364 us).
+constexpr int kFwdBatch = 4;
+
+template <class VT, bool HV, bool IN_H, bool CONTRACT>
+__global__ void __launch_bounds__(256, 6) spmm_fwd_kernel(SpmmParams p) {
+  __shared__ double sh[32];
+  const int P = p.nCh / (int)(sizeof(VT) / sizeof(float2));
+  const long long i0 = (long long)blockIdx.x * p.rows_per_block;
+  const int nr = (int)min((long long)p.rows_per_block, (long long)p.l_size - i0);
+  const int total = nr * P;
+  using In = GridIn<VT, IN_H>;
+  const typename In::T* in = reinterpret_cast<const typename In::T*>(p.in.a);
+  const float hin = IN_H ? 1.f / half_store_scale(p.in_h_amax, p.in_h_len) : 1.f;  // a power of two
+  double sq = 0.0;
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    const int lr = it / P, pi = it - lr * P;
+    const long long r = i0 + lr;
+    uint32_t k = __ldg(p.row_ptr + r);
+    const uint32_t e = __ldg(p.row_ptr + r + 1);
+    if (e - k > (uint32_t)kLongRow) continue;  // segment kernels own it
+    VT acc = vzero<VT>();
+    const typename In::T* const src = in + pi;
+    auto add = [&](float mm, VT vv) {
+      if constexpr (CONTRACT)
+        fma_to(acc, mm, vv);
+      else
+        acc = mul_add_rn(acc, mm, vv);
+    };
+    for (; k + kFwdBatch <= e; k += kFwdBatch) {
+      int j[kFwdBatch];
+      VT v[kFwdBatch];
+      float m[kFwdBatch];
+#pragma unroll
+      for (int q = 0; q < kFwdBatch; ++q) j[q] = __ldg(p.col + k + q);
+#pragma unroll
+      for (int q = 0; q < kFwdBatch; ++q) v[q] = In::at(src + (long long)j[q] * P, hin);
+#pragma unroll
+      for (int q = 0; q < kFwdBatch; ++q) m[q] = HV ? __half2float(p.val_h[k + q]) : __ldg(p.val + k + q);
+#pragma unroll
+      for (int q = 0; q < kFwdBatch; ++q) add(m[q], v[q]);
+    }
+    for (; k < e; ++k)
+      add(HV ? __half2float(p.val_h[k]) : __ldg(p.val + k), In::at(src + (long long)__ldg(p.col + k) * P, hin));
+    reinterpret_cast<VT*>(p.out.a)[r * P + pi] = acc;
+    if (p.partial) {
+      const double w = p.sqn_w ? (double)__ldg(p.sqn_w + r) : 1.0;
+      sq += w * sqnorm(acc);
+    }
+  }
   if (p.partial) {
     const double t = block_sum(sq, sh);
-    if (threadIdx.x == 0) p.partial[bid] = t;
+    if (threadIdx.x == 0) p.partial[blockIdx.x] = t;
   }
-}
-
-template <int PPT>
-static void launch_pair_ppt(bool contract, const SpmmParams& p, const int* rows, const uint2* rp, int nrows, int grid,
-                            const MidRows& mid, cudaStream_t s) {
-  grid += mid.blocks;
-  if (p.in_h_amax)  // FP16 input: contracted operator products only (checked by spmm)
-    spmm_pair_kernel<true, PPT, true><<<grid, 256, 0, s>>>(p, rows, rp, nrows, mid);
-  else if (contract)
-    spmm_pair_kernel<true, PPT><<<grid, 256, 0, s>>>(p, rows, rp, nrows, mid);
-  else
-    spmm_pair_kernel<false, PPT><<<grid, 256, 0, s>>>(p, rows, rp, nrows, mid);
-}
-
-static void launch_pair(int ppt, bool contract, const SpmmParams& p, const int* rows, const uint2* rp, int nrows,
-                        int grid, const MidRows& mid, cudaStream_t s) {
-  (void)ppt;  // one pair per thread (pair_ppt)
-  launch_pair_ppt<1>(contract, p, rows, rp, nrows, grid, mid, s);
 }
 
 // Short rows of an ordered non-empty product from their records (CONTRACT,
-// FP32 point layout in and out): a thread per (row, coil pair) reads the
-// row's 32-byte record -- cell, count and up to kRecInline (column, value)
-// pairs -- and issues every gather of the row at once, so such a row costs
-// two dependent loads (record -> inputs) instead of three (bounds -> entry ->
-// input), and the record stream is smaller than the bounds and entries it
-// replaces.  Rows with more entries loop over their CSR entries.  Per coil
-// the entries are summed in stored order with the same fused multiply-adds
-// as spmm_pair_kernel: the outputs are identical.  With FP16 matrix values
-// (p.val_h) the inline FP32 values are rounded to FP16 as they are read,
-// which gives the values the CSR rows read from val_h.  The first mid.blocks
-// blocks gather the mid rows a warp each, as there.  p.absmax (optional) is
-// raised to the largest output component.  Eight blocks per SM, as the pair
-// kernel.
-// (Loading two rows' records before either row's gathers -- two rows in
-// flight per thread at five blocks per SM, the registers of two records --
-// measured slower on c2: 0.709 against 0.610 ms.)
-template <bool HV, bool AM>
-__global__ void __launch_bounds__(256, 8) spmm_rec_kernel(SpmmParams p, const uint4* __restrict__ rec, int n_rows,
-                                                          MidRows mid) {
-  if ((int)blockIdx.x < mid.blocks) {
-    mid_rows_block<AM>(p, mid.rows, mid.bounds, mid.n, blockIdx.x, mid.blocks);
+// FP32 point layout in and out): a thread per (row, coil pair; VT = float2:
+// coil, for odd coil counts) reads the row's 32-byte record -- cell, count and
+// up to kRecInline (column, value) pairs -- and issues every gather of the
+// row at once, so such a row costs two dependent loads (record -> inputs)
+// instead of three (bounds -> entry -> input), and the record stream is
+// smaller than the bounds and entries it replaces.  Rows with more entries
+// loop over their CSR entries.  Per coil the entries are summed in stored
+// order with the same fused multiply-adds as spmm_pair_kernel: the outputs
+// are identical.  With FP16 matrix values (p.val_h) the inline FP32 values are
+// rounded to FP16 as they are read, which gives the values the CSR rows read
+// from val_h.  The first heavy.n blocks gather the heavy units, as there.
+// p.absmax (optional) is raised to the largest output component.
+//
+// Latency-bound gathers: the entries of longer rows go four at a time, as in
+// spmm_fwd_kernel, and a brick's rows are sorted by length (csr_build_order),
+// so that the rows of a warp (four at 16 coils) take one path.  MB resident
+// blocks per SM: six (40 registers), eight (32, a few spilled bytes) where the
+// k-space exceeds half the L2 and the gathers' latency grows (256^3 x 16
+// coils, 134 MB: 499 us at eight, 531 at six; 192^3 x 12 coils, 21 MB: 99 at
+// either, 512^2 x 12 coils 31 at six, 39 us at eight).  With the heavy units
+// in the launch Gut went from 606 to 499, 162 to 99, 122 to 59 (160 x 160 x
+// 120 x 8 coils) and 95 to 29 us.  (Measured and not kept: a warp's lanes
+// loading a row's entries together and passing them by shuffles, 512 and 124
+// us; two rows' records loaded before either row's gathers, 0.709 against
+// 0.610 ms then.)
+template <class VT, bool HV, bool AM, int MB>
+__global__ void __launch_bounds__(256, MB) spmm_rec_kernel(SpmmParams p, const uint4* __restrict__ rec, int n_rows,
+                                                           HeavyUnits heavy) {
+  if ((int)blockIdx.x < heavy.n) {
+    heavy_unit<VT, AM>(p, heavy, blockIdx.x);
     return;
   }
-  const int bid = (int)blockIdx.x - mid.blocks;
-  const int P = p.nCh >> 1;
+  const int bid = (int)blockIdx.x - heavy.n;
+  const int P = p.nCh / (int)(sizeof(VT) / sizeof(float2));
   const long long i0 = (long long)bid * p.rows_per_block;
   const int nr = (int)min((long long)p.rows_per_block, (long long)n_rows - i0);
   const int total = nr * P;
   const bool scale = p.in_row_scale != nullptr;
-  const float4* in = reinterpret_cast<const float4*>(p.in.a);
+  const VT* in = reinterpret_cast<const VT*>(p.in.a);
   float amax = 0.f;
   auto row = [&](const uint4 h0, const uint4 h1, const int pi) {
     const long long r = (int)h0.x;
     const uint32_t n = h0.y;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto fma4 = [&](float m, float4 v) {
-      acc.x = __fmaf_rn(m, v.x, acc.x);
-      acc.y = __fmaf_rn(m, v.y, acc.y);
-      acc.z = __fmaf_rn(m, v.z, acc.z);
-      acc.w = __fmaf_rn(m, v.w, acc.w);
-    };
+    VT acc = vzero<VT>();
     if (n <= (uint32_t)kRecInline) {
       const uint32_t c0 = h0.z, c1 = h1.x, c2 = h1.z;
-      float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0, v2 = v0;
+      VT v0 = vzero<VT>(), v1 = v0, v2 = v0;
       float m0 = __uint_as_float(h0.w), m1 = __uint_as_float(h1.y), m2 = __uint_as_float(h1.w);
       if constexpr (HV) {  // FP16 matrix values: the inline FP32 values rounded alike
         m0 = __half2float(__float2half_rn(m0));
@@ -531,24 +598,53 @@ __global__ void __launch_bounds__(256, 8) spmm_rec_kernel(SpmmParams p, const ui
         if (n > 1) m1 = __fmul_rn(m1, __ldg(p.in_row_scale + c1));
         if (n > 2) m2 = __fmul_rn(m2, __ldg(p.in_row_scale + c2));
       }
-      if (n > 0) fma4(m0, v0);
-      if (n > 1) fma4(m1, v1);
-      if (n > 2) fma4(m2, v2);
+      if (n > 0) fma_to(acc, m0, v0);
+      if (n > 1) fma_to(acc, m1, v1);
+      if (n > 2) fma_to(acc, m2, v2);
     } else {
-      const uint32_t b = h0.z;
-#pragma unroll 4
-      for (uint32_t k = b; k < b + n; ++k) {
-        const int j = __ldg(p.col + k);
-        float m = HV ? __half2float(p.val_h[k]) : __ldg(p.val + k);
-        const float4 v = __ldg(in + (long long)j * P + pi);
-        if (scale) m = __fmul_rn(m, __ldg(p.in_row_scale + j));
-        fma4(m, v);
+      constexpr int U = 4;
+      const VT* const src = in + pi;
+      uint32_t k = h0.z;
+      const uint32_t e = k + n;
+      for (; k + U <= e; k += U) {
+        int j[U];
+        float m[U];
+        VT v[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) j[q] = __ldg(p.col + k + q);
+#pragma unroll
+        for (int q = 0; q < U; ++q) v[q] = __ldg(src + (long long)j[q] * P);
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          m[q] = HV ? __half2float(p.val_h[k + q]) : __ldg(p.val + k + q);
+          if (scale) m[q] = __fmul_rn(m[q], __ldg(p.in_row_scale + j[q]));
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) fma_to(acc, m[q], v[q]);
+      }
+      if (k < e) {  // up to three more
+        int j[U - 1];
+        float m[U - 1];
+        VT v[U - 1];
+#pragma unroll
+        for (int q = 0; q < U - 1; ++q) j[q] = k + q < e ? __ldg(p.col + k + q) : -1;
+#pragma unroll
+        for (int q = 0; q < U - 1; ++q) {
+          v[q] = vzero<VT>();
+          m[q] = 0.f;
+          if (j[q] >= 0) {
+            v[q] = __ldg(src + (long long)j[q] * P);
+            m[q] = HV ? __half2float(p.val_h[k + q]) : __ldg(p.val + k + q);
+            if (scale) m[q] = __fmul_rn(m[q], __ldg(p.in_row_scale + j[q]));
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < U - 1; ++q)
+          if (j[q] >= 0) fma_to(acc, m[q], v[q]);
       }
     }
-    if (p.out_scale != 1.0f)
-      acc = make_float4(__fmul_rn(acc.x, p.out_scale), __fmul_rn(acc.y, p.out_scale), __fmul_rn(acc.z, p.out_scale),
-                        __fmul_rn(acc.w, p.out_scale));
-    reinterpret_cast<float4*>(p.out.a)[r * P + pi] = acc;
+    if (p.out_scale != 1.0f) acc = scaled(acc, p.out_scale);
+    reinterpret_cast<VT*>(p.out.a)[r * P + pi] = acc;
     if constexpr (AM) amax = fmaxf(amax, abs_max4(acc));
   };
   for (int it = threadIdx.x; it < total; it += blockDim.x) {
@@ -557,6 +653,66 @@ __global__ void __launch_bounds__(256, 8) spmm_rec_kernel(SpmmParams p, const ui
     row(__ldg(rp), __ldg(rp + 1), it - lr * P);
   }
   if constexpr (AM) block_absmax(p.absmax, amax);
+}
+
+// Rows per block of spmm_rec_kernel: a quarter of a brick's non-empty rows or
+// so (rows of neighbouring cells share samples in L1), more for the large
+// k-spaces, fewer where that would leave resident blocks without work.
+// Measured on 192^3 x 12, 160^2 x 120 x 8 and 512^2 x 12 coils: 64 rows 109 /
+// 64 / 29, 128 rows 99 / 58 / 36, 192 rows 99 / 63 / 46 us; on 256^3 x 16: 96
+// rows 521, 128 511, 192 499 us.
+static int rec_rows_per_block(int n_rows, int P, bool large) {
+  const int rows = std::min(large ? 192 : 128, n_rows / (148 * 24));
+  return std::max(rows, (256 + P - 1) / P);
+}
+
+template <class VT, bool HV, bool AM>
+static void launch_rec(const SpmmParams& p, const uint4* rec, int n_rows, const HeavyUnits& heavy, bool large,
+                       cudaStream_t s) {
+  SpmmParams q = p;
+  q.rows_per_block = rec_rows_per_block(n_rows, p.nCh / (int)(sizeof(VT) / sizeof(float2)), large);
+  const int g = heavy.n + (n_rows + q.rows_per_block - 1) / q.rows_per_block;
+  if (g == 0) return;
+  if (large)
+    spmm_rec_kernel<VT, HV, AM, 8><<<g, 256, 0, s>>>(q, rec, n_rows, heavy);
+  else
+    spmm_rec_kernel<VT, HV, AM, 6><<<g, 256, 0, s>>>(q, rec, n_rows, heavy);
+}
+
+template <class VT>
+static void launch_rec(const SpmmParams& p, const Csr& m, const HeavyUnits& heavy, cudaStream_t s) {
+  const uint4* rec = reinterpret_cast<const uint4*>(m.ord_rec);
+  const bool large = (size_t)m.r_size * p.nCh * sizeof(float2) > (64u << 20);  // half the L2
+  if (p.val_h)
+    p.absmax ? launch_rec<VT, true, true>(p, rec, m.ord_short, heavy, large, s)
+             : launch_rec<VT, true, false>(p, rec, m.ord_short, heavy, large, s);
+  else
+    p.absmax ? launch_rec<VT, false, true>(p, rec, m.ord_short, heavy, large, s)
+             : launch_rec<VT, false, false>(p, rec, m.ord_short, heavy, large, s);
+}
+
+// Whether a product runs as spmm_fwd_kernel: complex point layout, all rows in
+// row order, no scales, no recorded maximum.
+static bool use_fwd_kernel(const SpmmArgs& a) {
+  return a.in.layout == Layout::kPointC64 && a.out.layout == Layout::kPointC64 && !a.normalize &&
+         (a.contract || !a.half_values) && !a.nonempty_only && !a.long_only && !a.in_row_scale && a.out_scale == 1.0f && !a.absmax &&
+         !(a.m->ord_rows && !a.m->ord_nonempty);
+}
+
+static void launch_fwd(const SpmmParams& p, bool contract, int grid, cudaStream_t s) {
+  if (!contract) {
+    p.nCh % 2 ? spmm_fwd_kernel<float2, false, false, false><<<grid, 256, 0, s>>>(p)
+              : spmm_fwd_kernel<float4, false, false, false><<<grid, 256, 0, s>>>(p);
+  } else if (p.nCh % 2) {
+    p.val_h ? spmm_fwd_kernel<float2, true, false, true><<<grid, 256, 0, s>>>(p)
+            : spmm_fwd_kernel<float2, false, false, true><<<grid, 256, 0, s>>>(p);
+  } else if (p.in_h_amax) {
+    p.val_h ? spmm_fwd_kernel<float4, true, true, true><<<grid, 256, 0, s>>>(p)
+            : spmm_fwd_kernel<float4, false, true, true><<<grid, 256, 0, s>>>(p);
+  } else {
+    p.val_h ? spmm_fwd_kernel<float4, true, false, true><<<grid, 256, 0, s>>>(p)
+            : spmm_fwd_kernel<float4, false, false, true><<<grid, 256, 0, s>>>(p);
+  }
 }
 
 __global__ void rec_build_kernel(const int* __restrict__ rows, const uint2* __restrict__ bounds, int n,
@@ -601,22 +757,15 @@ int csr_build_records(Csr& c, cudaStream_t s) {
   return MLG_OK;
 }
 
-static bool use_pair_kernel(const SpmmArgs& a) {
-  return a.in.layout == Layout::kPointC64 &&
-         a.out.layout == Layout::kPointC64 && (a.nCh % 2) == 0 &&
-         !a.normalize;
+// complex point layout in and out, whole coil pairs
+static bool point_pairs(const SpmmArgs& a) {
+  return a.in.layout == Layout::kPointC64 && a.out.layout == Layout::kPointC64 && (a.nCh % 2) == 0 && !a.normalize;
 }
 
-// Coil pairs per thread of the pair kernel, as measured on a B200: one.
-// With eight 256-thread blocks per SM (32 registers) one pair per thread
-// matched two on the 4096 x 256-sample 16-coil Gu (0.381 vs 0.379 ms) and
-// beat it on a 1500-spoke one (0.164 vs 0.174 ms); at lower occupancy two
-// pairs had helped only that 16-coil Gu and slowed 12- and 8-coil products
-// and the non-empty-row Gut.
-static int pair_ppt(const SpmmArgs&) { return 1; }
+static bool use_pair_kernel(const SpmmArgs& a) { return point_pairs(a) && a.contract && !a.partial; }
 
 static int rows_per_block(const SpmmArgs& a) {
-  if (use_pair_kernel(a)) return std::max(1, 1024 / (a.nCh / 2 / pair_ppt(a)));
+  if (point_pairs(a)) return std::max(1, 1024 / (a.nCh / 2));
   return std::max(1, 1024 / std::max(1, a.nCh));
 }
 
@@ -627,7 +776,16 @@ int spmm_partial_count(const SpmmArgs& a) {
   return (int)((spmm_rows(a) + rpb - 1) / rpb) + a.m->n_long;
 }
 
-size_t spmm_scratch_floats(const Csr& m, int nCh) { return 3 * (size_t)m.n_seg * (size_t)nCh; }
+size_t spmm_scratch_floats(const Csr& m, int nCh) {
+  return std::max(3 * (size_t)m.n_seg, 2 * (size_t)m.n_multi_units) * (size_t)nCh;
+}
+
+// Odd coil counts: the ordered non-empty product by one coil per thread.
+static bool use_single_rec(const SpmmArgs& a) {
+  return a.in.layout == Layout::kPointC64 && a.out.layout == Layout::kPointC64 && (a.nCh % 2) == 1 && a.nCh <= 32 &&
+         a.nonempty_only && a.contract && !a.partial && !a.normalize && a.unit_count && a.m->ord_rec &&
+         a.m->ord_nonempty && a.m->ord_short >= 0;
+}
 
 template <Layout IN, Layout OUT, bool ROW_FAST>
 static int launch(const SpmmParams& p, const Csr& m, float3* scratch, int grid_short, cudaStream_t s) {
@@ -642,6 +800,16 @@ static int launch(const SpmmParams& p, const Csr& m, float3* scratch, int grid_s
     MLG_LAUNCHED();
   }
   return MLG_OK;
+}
+
+static HeavyUnits heavy_of(const Csr& m, float* scratch, unsigned* count) {
+  HeavyUnits h;
+  h.units = m.heavy_units;
+  h.multi = m.heavy_multi;
+  h.n = m.n_units;
+  h.scratch = scratch;
+  h.count = count;
+  return h;
 }
 
 int spmm(const SpmmArgs& a, cudaStream_t s) {
@@ -668,9 +836,9 @@ int spmm(const SpmmArgs& a, cudaStream_t s) {
   p.absmax = a.absmax;
   p.in_h_amax = a.in_half_amax;
   p.in_h_len = a.in_half_len;
-  MLG_CHECK(!a.in_half_amax || (use_pair_kernel(a) && a.contract && m.n_long == 0 && !a.nonempty_only),
-            "FP16 input: contracted coil-pair products without long rows only");
-  MLG_CHECK(!a.nonempty_only || (m.ord_rows && m.ord_nonempty && use_pair_kernel(a)),
+  MLG_CHECK(!a.in_half_amax || (use_fwd_kernel(a) && a.nCh % 2 == 0 && m.n_long == 0),
+            "FP16 input: forward coil-pair products without long rows only");
+  MLG_CHECK(!a.nonempty_only || (m.ord_rows && m.ord_nonempty && use_pair_kernel(a)) || use_single_rec(a),
             "non-empty-row products need the ordered row list and the coil-pair kernel");
   const long long nrows = spmm_rows(a);
   const int grid_all = (int)((nrows + p.rows_per_block - 1) / p.rows_per_block);
@@ -679,46 +847,50 @@ int spmm(const SpmmArgs& a, cudaStream_t s) {
   MLG_CHECK(m.n_long == 0 || m.n_seg > 0, "long rows without segment tables");
   DevBuf<float> own;
   float* scratch = a.seg_scratch;
-  if (m.n_long > 0 && !scratch) {
+  if ((m.n_long > 0 || m.n_multi_units > 0) && !scratch) {
     MLG_TRY(own.alloc(spmm_scratch_floats(m, a.nCh), s));
     scratch = own.p;
   }
   float3* sc3 = reinterpret_cast<float3*>(scratch);
   using L = Layout;
   const L i = a.in.layout, o = a.out.layout;
+  if (use_single_rec(a)) {
+    launch_rec<float2>(p, m, heavy_of(m, scratch, a.unit_count), s);
+    MLG_LAUNCHED();
+    return MLG_OK;
+  }
+  if (use_fwd_kernel(a) && grid_short > 0) {
+    launch_fwd(p, a.contract, grid_short, s);
+    MLG_LAUNCHED();
+    return launch<L::kPointC64, L::kPointC64, false>(p, m, sc3, 0, s);  // long rows
+  }
   if (use_pair_kernel(a)) {
     if (grid_short > 0) {
       // the matrix's processing order when it covers the requested rows
       const bool ordered = m.ord_rows && m.ord_nonempty == a.nonempty_only;
       MLG_CHECK(ordered || !a.nonempty_only, "non-empty-row products need the ordered row list");
-      // operator products over a split order: the short rows by the pair
-      // kernel, the longer ones by a warp each
-      const bool split = ordered && a.contract && m.ord_short >= 0 && !a.partial && a.nCh / 2 <= 16;
+      // operator products over a split order: the short rows by the record
+      // or pair kernel, the heavy ones as units in its first blocks
+      const bool split =
+          ordered && a.contract && m.ord_short >= 0 && !a.partial && a.nCh / 2 <= 16 && a.unit_count != nullptr;
       const int n_pair = split ? m.ord_short : (int)nrows;
-      MidRows mid;
-      if (split && nrows > n_pair) {  // about two mid rows per warp
-        mid.rows = m.ord_rows + n_pair;
-        mid.bounds = m.ord_bounds + n_pair;
-        mid.n = (int)nrows - n_pair;
-        mid.blocks = (mid.n + 15) / 16;
-      }
+      HeavyUnits heavy;
+      if (split) heavy = heavy_of(m, scratch, a.unit_count);
       const int grid_pair = split ? (n_pair + p.rows_per_block - 1) / p.rows_per_block : grid_short;
       const bool recs = records_forced() >= 0 ? records_forced() == 1 : a.records;
-      if (split && m.ord_rec && recs && grid_pair + mid.blocks > 0) {
-        const uint4* rec = reinterpret_cast<const uint4*>(m.ord_rec);
-        const int g = grid_pair + mid.blocks;
-        if (p.val_h)
-          p.absmax ? spmm_rec_kernel<true, true><<<g, 256, 0, s>>>(p, rec, n_pair, mid)
-                   : spmm_rec_kernel<true, false><<<g, 256, 0, s>>>(p, rec, n_pair, mid);
-        else
-          p.absmax ? spmm_rec_kernel<false, true><<<g, 256, 0, s>>>(p, rec, n_pair, mid)
-                   : spmm_rec_kernel<false, false><<<g, 256, 0, s>>>(p, rec, n_pair, mid);
+      if (split && m.ord_rec && recs) {
+        launch_rec<float4>(p, m, heavy, s);
         MLG_LAUNCHED();
-      } else if (grid_pair + mid.blocks > 0) {
-        launch_pair(pair_ppt(a), a.contract, p, ordered ? m.ord_rows : nullptr,
-                    ordered ? m.ord_bounds : nullptr, n_pair, grid_pair, mid, s);
+      } else if (grid_pair + heavy.n > 0) {
+        const int* rows = ordered ? m.ord_rows : nullptr;
+        const uint2* bounds = ordered ? m.ord_bounds : nullptr;
+        if (heavy.n)
+          spmm_pair_kernel<true><<<heavy.n + grid_pair, 256, 0, s>>>(p, rows, bounds, n_pair, heavy);
+        else
+          spmm_pair_kernel<false><<<grid_pair, 256, 0, s>>>(p, rows, bounds, n_pair, heavy);
         MLG_LAUNCHED();
       }
+      if (split) return MLG_OK;  // the heavy units hold the long rows
     }
     // long rows (segment kernels) with the same element types
     return launch<L::kPointC64, L::kPointC64, false>(p, m, sc3, 0, s);

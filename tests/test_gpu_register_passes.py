@@ -99,3 +99,35 @@ def test_solver_partial_sums():
         out.append(rec.run_host(y, np.ones(rec.nPt), nIter=1, nCGD=6, ve_max=1.0))
     assert rel(out[0], out[1]) <= 1e-5  # six steps of a few 1e-6 each at most
     rec.plan.close()
+
+
+@pytest.mark.parametrize("nCh", [1, 2, 3, 12, 16, 33])
+def test_gut_rows_of_every_length(nCh):
+    """The adjoint product over rows of 1 to several thousand entries: inline
+    records, loops with every remainder, rows of one heavy unit, rows of several
+    (the last unit to finish adds them; twice, so that the counters are seen
+    reset), against the product of every row (variant full_grid, no records).
+    Rows of n entries summed in another order: 6e-8 sqrt(n), n <= 4096 -> 4e-6."""
+    import torch
+
+    import monalisa_b200 as mb
+
+    rng = np.random.default_rng(nCh)
+    N = 32
+    # clusters of samples at one grid point: their 9 cells get rows of that many entries
+    sizes = list(range(1, 14)) + [16, 17, 63, 64, 65, 66, 255, 256, 257, 300, 513, 1500, 4000]
+    t = np.concatenate([np.repeat(np.array([[(3 * (i % 10)) - 14.0], [(3 * (i // 10)) - 14.0]]), n, 1)
+                        for i, n in enumerate(sizes)], 1) + rng.uniform(-0.2, 0.2, (2, sum(sizes)))
+    Gu, Gut = mb.bmTraj2SparseMat(t, np.ones(t.shape[1]), [N, N], [1, 1])
+    C = (rng.standard_normal((256, nCh)) + 1j * rng.standard_normal((256, nCh))).astype(np.complex64)
+    rec = mb.SensaRecon(Gu, Gut, C, [16, 16])
+    y = _cplx(rng, rec.nPt, nCh)
+    HY = torch.from_numpy(rng.random(rec.nPt).astype(np.float32)).cuda()
+    first = rec.plan.nakatsha(y, HY=HY, scale=3.0).cpu().numpy()
+    again = rec.plan.nakatsha(y, HY=HY, scale=3.0).cpu().numpy()
+    assert np.array_equal(first, again)
+    rec.plan.variant = {"pass_buffers": 0}
+    rec.plan.adjoint_mode = "full_grid"
+    ref = rec.plan.nakatsha(y, HY=HY, scale=3.0).cpu().numpy()
+    assert rel(first, ref) <= 4e-6, rel(first, ref)
+    rec.plan.close()
