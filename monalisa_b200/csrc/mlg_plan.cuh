@@ -78,7 +78,6 @@ struct mlg_plan_s {
   float dX[3] = {1.f, 1.f, 1.f};
   // captured inner CG step (replayed nCGD-1 times per outer iteration)
   cudaGraphExec_t cg_graph = nullptr;
-  const void* cg_graph_x = nullptr;  // solution buffer baked into the graph
   long long cg_graph_kernels = 0;
   // A plan created from another one (same grid, image, coils and KFC, other
   // matrices) borrows that plan's KFC, KFCc, grid, bufA, bufB, FFT tables,

@@ -17,12 +17,13 @@ namespace mlg {
 
 // device scalar slots
 enum : int {
-  S_SQN_CURR = 0,  // sqn_dagM_res_curr
-  S_SQN_MP = 1,
-  S_A = 2,
-  S_B = 3,
-  S_R = 4,         // monitoring residual
-  S_DONE = 5,      // 1.0 once sqn_curr < eps (inner loop stopped)
+  S_SQN_CURR = 0,  // sqn_dagM_res_curr of the running step
+  S_DONE = 1,      // 1.0 once sqn_curr < eps (inner loop stopped)
+  S_SQN_NEXT = 2,  // the same two for the step after it
+  S_DONE_NEXT = 3,
+  S_A = 4,
+  S_B = 5,
+  S_X = 6,         // address of the solution
   S_COUNT = 8
 };
 
@@ -95,23 +96,38 @@ __global__ void residual_kernel(const float2* __restrict__ y, const float2* __re
   }
 }
 
-// sqn_curr = HX * sum(partials); done = sqn_curr < eps   (bmSensa.m:45,54)
-__global__ void cg_init_kernel(const double* __restrict__ partial, int n, double HX, double eps, double* sc) {
+// sqn = HX * sum(partials); done = sqn < eps   (bmSensa.m:45,54); x: the
+// solution that the (captured) steps update
+__global__ void cg_init_kernel(const double* __restrict__ partial, int n, double HX, double eps, double* sc,
+                               float2* x, float2** x_slot) {
   __shared__ double sh[kT / 32];
   const double s = sum_partials(partial, n, sh);
   if (threadIdx.x == 0) {
-    sc[S_SQN_CURR] = HX * s;
-    sc[S_DONE] = (HX * s < eps) ? 1.0 : 0.0;
+    sc[S_SQN_NEXT] = HX * s;
+    sc[S_DONE_NEXT] = (HX * s < eps) ? 1.0 : 0.0;
+    *x_slot = x;
   }
 }
+
+// The scalars of a step are summed by every CTA of the update that needs them
+// (the same fixed order in each, so the same value) while the partials are at
+// most kFusedPartials; a scalar kernel and two updates take 3 to 4 us each
+// where the vectors are small, and the sum re-read by each CTA outweighs a
+// launch where there are thousands of partials.  The CTAs of a kernel read one
+// copy of (sqn, done) and CTA 0 writes the other: the alpha kernels NEXT ->
+// CURR, the beta kernels CURR -> NEXT.
+// 20 steps, 512^2 grid, 1 coil, another solution buffer on each call: 1.32 -> 1.10
+// ms with the three launches per step and the repeated capture gone.
+constexpr int kFusedPartials = 1024;
 
 // sqn_Mp = sum(partials); a = sqn_curr / sqn_Mp   (bmSensa.m:59-61)
 __global__ void cg_alpha_kernel(const double* __restrict__ partial, int n, double* sc) {
   __shared__ double sh[kT / 32];
   const double s = sum_partials(partial, n, sh);
   if (threadIdx.x == 0) {
-    sc[S_SQN_MP] = s;
-    sc[S_A] = sc[S_DONE] != 0.0 ? 0.0 : sc[S_SQN_CURR] / s;
+    sc[S_SQN_CURR] = sc[S_SQN_NEXT];
+    sc[S_DONE] = sc[S_DONE_NEXT];
+    sc[S_A] = sc[S_DONE_NEXT] != 0.0 ? 0.0 : sc[S_SQN_NEXT] / s;
   }
 }
 
@@ -120,13 +136,11 @@ __global__ void cg_alpha_kernel(const double* __restrict__ partial, int n, doubl
 __global__ void cg_beta_kernel(const double* __restrict__ partial, int n, double HX, double eps, double* sc) {
   __shared__ double sh[kT / 32];
   const double s = sum_partials(partial, n, sh);
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && sc[S_DONE] == 0.0) {
     const double next = HX * s;
-    if (sc[S_DONE] == 0.0) {
-      sc[S_B] = next / sc[S_SQN_CURR];
-      sc[S_SQN_CURR] = next;
-      if (next < eps) sc[S_DONE] = 1.0;
-    }
+    sc[S_B] = next / sc[S_SQN_CURR];
+    sc[S_SQN_NEXT] = next;
+    if (next < eps) sc[S_DONE_NEXT] = 1.0;
   }
 }
 
@@ -136,29 +150,48 @@ __global__ void sum_to_slot_kernel(const double* __restrict__ partial, int n, do
   if (threadIdx.x == 0) sc[slot] = s;
 }
 
-// x += a p   (bmSensa.m:63)
-__global__ void cg_update_x_kernel(float2* __restrict__ x, const float2* __restrict__ p, long long n,
-                                   const double* __restrict__ sc) {
-  if (sc[S_DONE] != 0.0) return;
-  const float a = (float)sc[S_A];
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+// x += a p (bmSensa.m:63); res -= a Mp (:71) unless res is null; FUSED: a
+// from the partials here.  The residual and M p are FP32 complex in
+// every precision (M p in scaled FP16 was measured: the store slowed the
+// latency-bound Gu gather by more than the halved k-space traffic saved, c2
+// mixed 97.3 against 95.6 ms, and raised the image error 1.06e-4 -> 1.33e-4)
+template <bool FUSED>
+__global__ void __launch_bounds__(kT) cg_update_kernel(float2* const* __restrict__ x_slot, const float2* __restrict__ p,
+                                                       long long nx, float2* __restrict__ res,
+                                                       const float2* __restrict__ Mp, long long nk, double* sc,
+                                                       const double* __restrict__ partial, int n) {
+  double ad;
+  if constexpr (FUSED) {
+    __shared__ double sh[kT / 32];
+    __shared__ double s_a;
+    const double done = sc[S_DONE_NEXT], sqn = sc[S_SQN_NEXT];
+    const double s = sum_partials(partial, n, sh);
+    if (threadIdx.x == 0) {
+      s_a = sqn / s;
+      if (blockIdx.x == 0) {
+        sc[S_SQN_CURR] = sqn;
+        sc[S_DONE] = done;
+      }
+    }
+    if (done != 0.0) return;
+    __syncthreads();
+    ad = s_a;
+  } else {
+    if (sc[S_DONE] != 0.0) return;
+    ad = sc[S_A];
+  }
+  const float a = (float)ad;
+  float2* x = *x_slot;
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  for (long long i = first; i < nx; i += step) {
     const float2 pv = p[i];
     float2 xv = x[i];
     xv.x = __fadd_rn(xv.x, __fmul_rn(a, pv.x));
     xv.y = __fadd_rn(xv.y, __fmul_rn(a, pv.y));
     x[i] = xv;
   }
-}
-
-// res -= a Mp   (bmSensa.m:71); the residual and M p are FP32 complex in
-// every precision (M p in scaled FP16 was measured: the store slowed the
-// latency-bound Gu gather by more than the halved k-space traffic saved, c2
-// mixed 97.3 against 95.6 ms, and raised the image error 1.06e-4 -> 1.33e-4)
-__global__ void cg_update_res_kernel(float2* __restrict__ res, const float2* __restrict__ Mp, long long n,
-                                     const double* __restrict__ sc) {
-  if (sc[S_DONE] != 0.0) return;
-  const float a = (float)sc[S_A];
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+  if (!res) return;
+  for (long long i = first; i < nk; i += step) {
     const float2 m = Mp[i];
     float2 r = res[i];
     r.x = __fsub_rn(r.x, __fmul_rn(a, m.x));
@@ -172,15 +205,55 @@ static void launch_residual(int g, const float2* y, const float2* Mx, long long 
   residual_kernel<<<g, kT, 0, s>>>(y, Mx, n, nCh, HY, res, partial);
 }
 
-// p = dagM + b p   (bmSensa.m:77)
-__global__ void cg_update_p_kernel(float2* __restrict__ p, const float2* __restrict__ dagM, long long n,
-                                   const double* __restrict__ sc) {
-  if (sc[S_DONE] != 0.0) return;
-  const float b = (float)sc[S_B];
+// p = dagM + b p   (bmSensa.m:77); FUSED: b from the partials here
+template <bool FUSED>
+__global__ void __launch_bounds__(kT) cg_update_p_kernel(float2* __restrict__ p, const float2* __restrict__ dagM,
+                                                         long long n, double* sc, const double* __restrict__ partial,
+                                                         int np, double HX, double eps) {
+  double bd;
+  if constexpr (FUSED) {
+    __shared__ double sh[kT / 32];
+    __shared__ double s_next;
+    const double curr = sc[S_SQN_CURR];
+    if (sc[S_DONE] != 0.0) return;  // NEXT already holds the same
+    const double s = sum_partials(partial, np, sh);
+    if (threadIdx.x == 0) {
+      const double next = HX * s;
+      s_next = next;
+      if (blockIdx.x == 0) {
+        sc[S_SQN_NEXT] = next;
+        if (next < eps) sc[S_DONE_NEXT] = 1.0;
+      }
+    }
+    __syncthreads();
+    if (s_next < eps) return;
+    bd = s_next / curr;
+  } else {
+    if (sc[S_DONE_NEXT] != 0.0) return;
+    bd = sc[S_B];
+  }
+  const float b = (float)bd;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const float2 d = dagM[i], pv = p[i];
     p[i] = make_float2(__fadd_rn(d.x, __fmul_rn(b, pv.x)), __fadd_rn(d.y, __fmul_rn(b, pv.y)));
   }
+}
+
+static float2** x_slot(mlg_plan_s* p) { return reinterpret_cast<float2**>(p->scalars + S_X); }
+
+// x += a p and, with res, res -= a Mp, a from np partials
+static int cg_update(mlg_plan_s* p, int np, float2* res, cudaStream_t s) {
+  const long long nk = res ? (long long)p->nPt * p->nCh : 0;
+  const int g = grid1(std::max<long long>(p->nu_tot, nk));
+  if (np <= kFusedPartials) {
+    cg_update_kernel<true><<<g, kT, 0, s>>>(x_slot(p), p->x_p, p->nu_tot, res, p->k_Mp, nk, p->scalars, p->partial, np);
+  } else {
+    cg_alpha_kernel<<<1, kT, 0, s>>>(p->partial, np, p->scalars);
+    MLG_LAUNCHED();
+    cg_update_kernel<false><<<g, kT, 0, s>>>(x_slot(p), p->x_p, p->nu_tot, res, p->k_Mp, nk, p->scalars, nullptr, 0);
+  }
+  MLG_LAUNCHED();
+  return MLG_OK;
 }
 
 static int ensure_solver_buffers(mlg_plan_s* p) {
@@ -206,20 +279,19 @@ static int ensure_solver_buffers(mlg_plan_s* p) {
 }
 
 // One inner CG step i < nCGD (bmSensa.m:50-77 without the final break).
-static int cg_step(mlg_plan_s* p, float2* x, double HX, double eps, cudaStream_t s) {
-  const long long nk = (long long)p->nPt * p->nCh;
+static int cg_step(mlg_plan_s* p, double HX, double eps, cudaStream_t s) {
   int np = 0;
   MLG_TRY(shanna_run(p, p->x_p, false, p->k_Mp, p->HY, p->partial, &np, s));
-  cg_alpha_kernel<<<1, kT, 0, s>>>(p->partial, np, p->scalars);
-  MLG_LAUNCHED();
-  cg_update_x_kernel<<<grid1(p->nu_tot), kT, 0, s>>>(x, p->x_p, p->nu_tot, p->scalars);
-  MLG_LAUNCHED();
-  cg_update_res_kernel<<<grid1(nk), kT, 0, s>>>(p->k_res, p->k_Mp, nk, p->scalars);
-  MLG_LAUNCHED();
+  MLG_TRY(cg_update(p, np, p->k_res, s));
   MLG_TRY(nakatsha_run(p, p->k_res, p->HY, (float)(1.0 / HX), p->x_dagM, p->partial, &np, s));
-  cg_beta_kernel<<<1, kT, 0, s>>>(p->partial, np, HX, eps, p->scalars);
-  MLG_LAUNCHED();
-  cg_update_p_kernel<<<grid1(p->nu_tot), kT, 0, s>>>(p->x_p, p->x_dagM, p->nu_tot, p->scalars);
+  const int g = grid1(p->nu_tot);
+  if (np <= kFusedPartials) {
+    cg_update_p_kernel<true><<<g, kT, 0, s>>>(p->x_p, p->x_dagM, p->nu_tot, p->scalars, p->partial, np, HX, eps);
+  } else {
+    cg_beta_kernel<<<1, kT, 0, s>>>(p->partial, np, HX, eps, p->scalars);
+    MLG_LAUNCHED();
+    cg_update_p_kernel<false><<<g, kT, 0, s>>>(p->x_p, p->x_dagM, p->nu_tot, p->scalars, nullptr, 0, HX, eps);
+  }
   MLG_LAUNCHED();
   return MLG_OK;
 }
@@ -261,18 +333,20 @@ static int sensa_body(mlg_plan_s* p, const float2* y, const float* ve, float ve_
   MLG_LAUNCHED();
 
   const int full = std::max(0, nCGD - 1);  // inner steps that run to p_next
-  // Captured once per solution buffer, after the first init phase has run
-  // every kernel of the step at least once (first launches set kernel
-  // attributes, which must not happen during capture).
+  // Captured once, after the first init phase has run every transform and
+  // product kernel of the step (first launches set kernel attributes, which
+  // must not happen during capture).  The step reads the solution's address
+  // from x_slot, set by cg_init_kernel: a graph that holds it was captured
+  // again on each call with another buffer.
   auto ensure_graph = [&]() -> int {
-    if (!use_graph || full == 0 || (p->cg_graph && p->cg_graph_x == x && p->cg_graph_prec == (int)p->mixed_run))
+    if (!use_graph || full == 0 || (p->cg_graph && p->cg_graph_prec == (int)p->mixed_run))
       return MLG_OK;
     if (p->cg_graph) cudaGraphExecDestroy(p->cg_graph);
     p->cg_graph = nullptr;
     cudaGraph_t graph;
     MLG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     const long long before = g_launches.load();
-    const int st = cg_step(p, x, HX, eps, s);
+    const int st = cg_step(p, HX, eps, s);
     const cudaError_t ce = cudaStreamEndCapture(s, &graph);
     p->cg_graph_kernels = g_launches.load() - before;
     g_launches.fetch_sub(p->cg_graph_kernels);  // captured, not launched
@@ -281,7 +355,6 @@ static int sensa_body(mlg_plan_s* p, const float2* y, const float* ve, float ve_
     const cudaError_t ie = cudaGraphInstantiate(&p->cg_graph, graph, 0);
     cudaGraphDestroy(graph);
     if (ie != cudaSuccess) return fail(MLG_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ie));
-    p->cg_graph_x = x;
     p->cg_graph_prec = (int)p->mixed_run;
     return MLG_OK;
   };
@@ -296,7 +369,7 @@ static int sensa_body(mlg_plan_s* p, const float2* y, const float* ve, float ve_
     launch_residual(grid1(nk), y, p->k_Mp, nk, p->nCh, p->HY, p->k_res, nullptr, s);
     MLG_LAUNCHED();
     MLG_TRY(nakatsha_run(p, p->k_res, p->HY, (float)(1.0 / HX), p->x_dagM, p->partial, &np, s));
-    cg_init_kernel<<<1, kT, 0, s>>>(p->partial, np, HX, eps, p->scalars);
+    cg_init_kernel<<<1, kT, 0, s>>>(p->partial, np, HX, eps, p->scalars, x, x_slot(p));
     MLG_LAUNCHED();
     MLG_CUDA(cudaMemcpyAsync(p->x_p, p->x_dagM, sizeof(float2) * (size_t)p->nu_tot, cudaMemcpyDeviceToDevice, s));
     p->cg_half = p->mixed_run;  // the CG steps: FP16 transform intermediate where supported
@@ -306,15 +379,12 @@ static int sensa_body(mlg_plan_s* p, const float2* y, const float* ve, float ve_
         MLG_CUDA(cudaGraphLaunch(p->cg_graph, s));
         count_launch(p->cg_graph_kernels);
       } else {
-        MLG_TRY(cg_step(p, x, HX, eps, s));
+        MLG_TRY(cg_step(p, HX, eps, s));
       }
     }
     if (nCGD > 0) {  // the last step stops after x += a p (bmSensa.m:67-69)
       MLG_TRY(shanna_run(p, p->x_p, false, p->k_Mp, p->HY, p->partial, &np, s));
-      cg_alpha_kernel<<<1, kT, 0, s>>>(p->partial, np, p->scalars);
-      MLG_LAUNCHED();
-      cg_update_x_kernel<<<grid1(p->nu_tot), kT, 0, s>>>(x, p->x_p, p->nu_tot, p->scalars);
-      MLG_LAUNCHED();
+      MLG_TRY(cg_update(p, np, nullptr, s));
     }
     // monitoring: R = |y - Mx|^2_HY   (bmSensa.m:82-83)
     p->cg_half = false;
@@ -347,6 +417,10 @@ int mlg_plan_set_dk(mlg_plan_t p, const double* dK_u) {
     // single-precision arithmetic of bmSensa.m:26-27
     dx[d] = (1.0f / (float)dK_u[d]) / (float)p->N[d];
     hx = (double)((float)hx * dx[d]);
+  }
+  if (p->HX != hx && p->cg_graph) {  // captured with the other HX
+    cudaGraphExecDestroy(p->cg_graph);
+    p->cg_graph = nullptr;
   }
   p->HX = hx;
   for (int d = 0; d < 3; ++d) p->dX[d] = dx[d];
@@ -448,7 +522,6 @@ extern "C" int mlg_plan_set_adjoint(mlg_plan_t p, int mode) {
     p->adjoint_mode = mode;
     if (p->cg_graph) cudaGraphExecDestroy(p->cg_graph);  // captured with the old strategy
     p->cg_graph = nullptr;
-    p->cg_graph_x = nullptr;
   }
   return MLG_OK;
 }
@@ -518,7 +591,6 @@ extern "C" int mlg_plan_set_variant(mlg_plan_t p, int pass_buffers, int gut_reco
     p->fwd_masked_store = fwd_masked_store;
     if (p->cg_graph) cudaGraphExecDestroy(p->cg_graph);  // captured with the old kernels
     p->cg_graph = nullptr;
-    p->cg_graph_x = nullptr;
   }
   return MLG_OK;
 }
@@ -530,7 +602,6 @@ extern "C" int mlg_plan_set_register_passes(mlg_plan_t p, int on) {
     p->reg_passes = on;
     if (p->cg_graph) cudaGraphExecDestroy(p->cg_graph);  // captured with the other kernels
     p->cg_graph = nullptr;
-    p->cg_graph_x = nullptr;
   }
   return MLG_OK;
 }
@@ -662,7 +733,6 @@ extern "C" int mlg_plan_set_precision(mlg_plan_t p, int precision) {
     p->adjoint_mode = adjoint_mode_valid(p, 2) ? 2 : 0;
   if (p->cg_graph) cudaGraphExecDestroy(p->cg_graph);
   p->cg_graph = nullptr;
-  p->cg_graph_x = nullptr;
   return MLG_OK;
 }
 
