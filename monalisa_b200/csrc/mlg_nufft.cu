@@ -690,6 +690,7 @@ static int plan_create_impl(int imDim, const int* N_u, const int* n_u, int nCh, 
     SpmmArgs a;
     a.m = &p->Gu_s;
     a.nCh = nCh;
+    a.in.layout = a.out.layout = Layout::kPointC64;  // as the solver's product
     cap = std::max(cap, spmm_partial_count(a));
   }
   cap = std::max(cap, ew_grid((long long)p->nPt * nCh) + 8);

@@ -764,12 +764,20 @@ static bool point_pairs(const SpmmArgs& a) {
 
 static bool use_pair_kernel(const SpmmArgs& a) { return point_pairs(a) && a.contract && !a.partial; }
 
-static int rows_per_block(const SpmmArgs& a) {
-  if (point_pairs(a)) return std::max(1, 1024 / (a.nCh / 2));
-  return std::max(1, 1024 / std::max(1, a.nCh));
-}
-
 static long long spmm_rows(const SpmmArgs& a) { return a.nonempty_only ? a.m->n_nonempty : a.m->l_size; }
+
+// Rows per CTA of the row-per-thread-group products: a thread's share is four
+// rows where there are enough of them, fewer where the CTAs would not fill
+// 148 SMs x 6 (a product's few hundred CTAs of four rows each are a chain of
+// dependent gathers on a part of the chip).  Gu of a 64^3 grid, 1 coil: 25 -> 12
+// us, 96^3 x 4 coils 25 -> 15, 256^2 x 8 coils 12.7 -> 8.6 (8 CG steps 444 -> 392),
+// 512^2 x 1 coil 12.8 -> 10.6 us; from 1.2 million (row, coil pair)s on the same.
+static int rows_per_block(const SpmmArgs& a) {
+  const int lanes = std::max(1, point_pairs(a) ? a.nCh / 2 : a.nCh);
+  const int least = std::max(1, 256 / lanes), most = std::max(1, 1024 / lanes);
+  const long long want = (spmm_rows(a) + 148 * 6 - 1) / (148 * 6);
+  return (int)std::min<long long>(most, (want + least - 1) / least * least);
+}
 
 int spmm_partial_count(const SpmmArgs& a) {
   const int rpb = rows_per_block(a);
