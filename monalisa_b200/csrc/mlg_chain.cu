@@ -67,8 +67,7 @@ struct mlg_chain_s {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
   cudaGraphExec_t graph = nullptr;
-  const void* graph_key[4] = {nullptr, nullptr, nullptr, nullptr};
-  std::vector<int> graph_modes;     // sparsifier and the frames' adjoint strategies it was captured with
+  std::vector<double> graph_modes;  // sparsifier, scales, the frames' adjoint strategies and kernels it was captured with
   long long graph_kernels = 0;
   // deformation fields of the temporal sparsifier (caller's matrices, one
   // per frame, NULL = identity): F x_f = Tu_f x_f - x_{f-1}, F* z_f =
@@ -93,6 +92,7 @@ enum : int {
   T_DAFI = 8,     // monitoring, latest
   T_REGUL = 9,
   T_ITER = 10,    // ADMM iteration index (0-based) the lists are read at
+  T_X = 11,       // address of the solution
   T_COUNT = 16
 };
 
@@ -165,7 +165,9 @@ __global__ void tv_scale_kernel(const float2* __restrict__ v, long long n, float
 // delta and rho of ADMM iteration T_ITER (:104-110): the lists, or in the
 // 'adapt' mode delta = delta_factor * regul / dafi, rho = rho_factor * delta
 // (private_adapt_delta_rho, :240-248)
-__global__ void tv_params_kernel(const double* __restrict__ lists, int cap, int adapt, double* sc) {
+__global__ void tv_params_kernel(const double* __restrict__ lists, int cap, int adapt, double* sc, float2* x,
+                                 float2** x_slot) {
+  *x_slot = x;
   const int c = (int)sc[T_ITER];
   const float dl = (float)lists[c], rl = (float)lists[cap + c];
   float d = dl, r = rl;
@@ -267,24 +269,37 @@ __global__ void tv_beta_kernel(const double* __restrict__ partial, int n, double
   }
 }
 
-// v += a w   (x update :147; res_y / res_z updates :154-155 with v -= a w)
-template <bool MINUS>
-__global__ void tv_axpy_kernel(float2* __restrict__ v, const float2* __restrict__ w, long long n,
-                               const double* __restrict__ sc) {
+// x += a p (:147) and, with res_y, res_y -= a Mp and res_z -= a Fp (:154-155):
+// one launch for the three (a few us each where the frames are small).  x's
+// address is read from device memory, so that the captured step serves every
+// solution buffer.
+__global__ void tv_update_kernel(float2* const* __restrict__ x_slot, const float2* __restrict__ p, long long nx,
+                                 float2* __restrict__ res_y, const float2* __restrict__ Mp, long long nk,
+                                 float2* __restrict__ res_z, const float2* __restrict__ Fp, long long nd,
+                                 const double* __restrict__ sc) {
   if (sc[T_DONE] != 0.0) return;
   const float a = (float)sc[T_A];
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float2 wv = w[i];
-    float2 x = v[i];
-    if (MINUS) {
-      x.x = __fsub_rn(x.x, __fmul_rn(a, wv.x));
-      x.y = __fsub_rn(x.y, __fmul_rn(a, wv.y));
-    } else {
-      x.x = __fadd_rn(x.x, __fmul_rn(a, wv.x));
-      x.y = __fadd_rn(x.y, __fmul_rn(a, wv.y));
-    }
-    v[i] = x;
+  float2* x = *x_slot;
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  for (long long i = first; i < nx; i += step) {
+    const float2 w = p[i];
+    float2 v = x[i];
+    v.x = __fadd_rn(v.x, __fmul_rn(a, w.x));
+    v.y = __fadd_rn(v.y, __fmul_rn(a, w.y));
+    x[i] = v;
   }
+  if (!res_y) return;
+  auto minus = [&](float2* r, const float2* m, long long n) {
+    for (long long i = first; i < n; i += step) {
+      const float2 w = m[i];
+      float2 v = r[i];
+      v.x = __fsub_rn(v.x, __fmul_rn(a, w.x));
+      v.y = __fsub_rn(v.y, __fmul_rn(a, w.y));
+      r[i] = v;
+    }
+  };
+  minus(res_y, Mp, nk);
+  minus(res_z, Fp, nd);
 }
 
 // p = dA + b p   (:161)
@@ -582,9 +597,14 @@ static int chain_dagA(mlg_chain_s* c, bool first, cudaStream_t s) {
   return MLG_OK;
 }
 
-// Le_Midi and Le_Soir: Mp, Fp, a, x += a p   (:138-147)
-static int chain_cg_half(mlg_chain_s* c, float2* x, cudaStream_t s) {
+static float2** x_slot(mlg_chain_s* c) { return reinterpret_cast<float2**>(c->sc + T_X); }
+
+// Le_Midi and Le_Soir: Mp, Fp, a, x += a p (:138-147); with residuals, those too
+// (:154-155)
+static int chain_cg_half(mlg_chain_s* c, bool residuals, cudaStream_t s) {
   const long long ni = c->nu * c->nFr;
+  const long long nk = residuals ? c->rows * c->nCh : 0;
+  const long long nd = residuals ? c->nu * (c->spatial ? c->geom.dim : c->nFr) : 0;
   int n_mp = 0;
   MLG_TRY(chain_forward(c, c->p, c->Mp, c->HY, &n_mp, s));
   const int g = grid1(ni);
@@ -599,19 +619,16 @@ static int chain_cg_half(mlg_chain_s* c, float2* x, cudaStream_t s) {
   MLG_LAUNCHED();
   tv_alpha_kernel<<<1, kT, 0, s>>>(c->partial, n_mp, g, c->HX, c->sc);
   MLG_LAUNCHED();
-  tv_axpy_kernel<false><<<grid1(ni), kT, 0, s>>>(x, c->p, ni, c->sc);
+  tv_update_kernel<<<grid1(std::max(ni, std::max(nk, nd))), kT, 0, s>>>(
+      x_slot(c), c->p, ni, residuals ? c->res_y : nullptr, c->Mp, nk, c->res_z, c->Fp, nd, c->sc);
   MLG_LAUNCHED();
   return MLG_OK;
 }
 
 // one full CG step j < nCGD (:128-161)
-static int chain_cg_step(mlg_chain_s* c, float2* x, cudaStream_t s) {
-  const long long ni = c->nu * c->nFr, nk = c->rows * c->nCh, nd = c->nu * (c->spatial ? c->geom.dim : c->nFr);
-  MLG_TRY(chain_cg_half(c, x, s));
-  tv_axpy_kernel<true><<<grid1(nk), kT, 0, s>>>(c->res_y, c->Mp, nk, c->sc);
-  MLG_LAUNCHED();
-  tv_axpy_kernel<true><<<grid1(nd), kT, 0, s>>>(c->res_z, c->Fp, nd, c->sc);
-  MLG_LAUNCHED();
+static int chain_cg_step(mlg_chain_s* c, cudaStream_t s) {
+  const long long ni = c->nu * c->nFr;
+  MLG_TRY(chain_cg_half(c, true, s));
   MLG_TRY(chain_dagA(c, false, s));
   tv_update_p_kernel<<<grid1(ni), kT, 0, s>>>(c->p, c->dA, ni, c->sc);
   MLG_LAUNCHED();
@@ -701,16 +718,17 @@ static int chain_run(mlg_chain_s* c, bool spatial, const float2* y, const float*
 
   const int full = std::max(0, nCGD - 1);
   auto ensure_graph = [&]() -> int {
-    const void* key[4] = {x, z, u, y};
-    std::vector<int> modes{spatial ? 1 : 0};
-    for (const mlg_plan_s* p : c->fr) modes.push_back(p->adjoint_mode);
-    if (full == 0 || (c->graph && std::equal(key, key + 4, c->graph_key) && modes == c->graph_modes)) return MLG_OK;
+    std::vector<double> modes{spatial ? 1.0 : 0.0, c->HX, c->geom.dX[0], c->geom.dX[1], c->geom.dX[2]};
+    for (const mlg_plan_s* p : c->fr)
+      for (int m : {p->adjoint_mode, p->reg_passes, p->pass_buffers, p->gut_records, p->fwd_masked_store, p->precision})
+        modes.push_back(m);
+    if (full == 0 || (c->graph && modes == c->graph_modes)) return MLG_OK;
     if (c->graph) cudaGraphExecDestroy(c->graph);
     c->graph = nullptr;
     cudaGraph_t g;
     MLG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     const long long before = g_launches.load();
-    const int st = chain_cg_step(c, x, s);
+    const int st = chain_cg_step(c, s);
     const cudaError_t ce = cudaStreamEndCapture(s, &g);
     c->graph_kernels = g_launches.load() - before;
     g_launches.fetch_sub(c->graph_kernels);  // captured, not launched
@@ -719,13 +737,12 @@ static int chain_run(mlg_chain_s* c, bool spatial, const float2* y, const float*
     const cudaError_t ie = cudaGraphInstantiate(&c->graph, g, 0);
     cudaGraphDestroy(g);
     if (ie != cudaSuccess) return fail(MLG_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ie));
-    std::copy(key, key + 4, c->graph_key);
     c->graph_modes = modes;
     return MLG_OK;
   };
 
   for (int it = 0; it < nIter; ++it) {
-    tv_params_kernel<<<1, 1, 0, s>>>(c->lists, c->lists_cap, adapt, c->sc);
+    tv_params_kernel<<<1, 1, 0, s>>>(c->lists, c->lists_cap, adapt, c->sc, x, x_slot(c));
     MLG_LAUNCHED();
     // L_Aube (:116-123): res_y is the kept monitoring residual
     if (spatial) {
@@ -744,7 +761,7 @@ static int chain_run(mlg_chain_s* c, bool spatial, const float2* y, const float*
       MLG_CUDA(cudaGraphLaunch(c->graph, s));
       count_launch(c->graph_kernels);
     }
-    if (nCGD > 0) MLG_TRY(chain_cg_half(c, x, s));  // the last step stops after x += a p (:148-150)
+    if (nCGD > 0) MLG_TRY(chain_cg_half(c, false, s));  // the last step stops after x += a p (:148-150)
     if (spatial) {
       st_zu_kernel<<<grid1(ni), kT, 0, s>>>(x, c->nu, c->geom, z, u, c->sc);
     } else {

@@ -46,3 +46,28 @@ def test_steps_replay_for_every_solution_buffer(N, n, nCh, spokes):
         assert torch.equal(torch.view_as_real(x), torch.view_as_real(xs[0]))
     assert float(xs[0].abs().max()) > 0
     rec.plan.close()
+
+
+def test_chain_step_replays_for_every_solution_buffer():
+    """The temporal chain's captured step, called with alternating x, z, u."""
+    import torch
+
+    import monalisa_b200 as mb
+
+    rng = np.random.default_rng(3)
+    N, n, nCh = [48, 40], [24, 20], 3
+    t = [(rng.random((2, m)) - 0.5) * 36 for m in (700, 911)]
+    mats = [mb.bmTraj2SparseMat(v, np.ones(v.shape[1]), N, [1, 1]) for v in t]
+    nu, rows = 480, 1611
+    C = (rng.standard_normal((nu, nCh)) + 1j * rng.standard_normal((nu, nCh))).astype(np.complex64)
+    chain = mb.TevaMorphosiaChain([m[0] for m in mats], [m[1] for m in mats], C, n)
+    y = torch.from_numpy((rng.standard_normal((rows, nCh)) + 1j * rng.standard_normal((rows, nCh))).astype(np.complex64)).cuda()
+    ve = torch.ones(rows, device="cuda")
+    bufs = [[torch.zeros((2, nu), dtype=torch.complex64, device="cuda") for _ in range(3)] for _ in range(3)]
+    for x, z, u in bufs:
+        chain.run_dev(y, ve, x, z, u, 0.01, 0.1, 2, 4, 1.0)
+    torch.cuda.synchronize()
+    for b in bufs[1:]:
+        for v, w in zip(b, bufs[0]):
+            assert torch.equal(torch.view_as_real(v), torch.view_as_real(w))
+    assert float(bufs[0][0].abs().max()) > 0
