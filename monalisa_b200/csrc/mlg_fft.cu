@@ -175,12 +175,13 @@ int fft_reg_group_6(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStr
 int fft_reg_group_7(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
 int fft_reg_group_8(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
 int fft_reg_group_9(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
+int fft_reg_group_10(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
 
 // The pass's register kernel; *done stays false where there is none.
 static int fft_reg_pass(const FftAxisPlan& a, PassMode mode, const PassDesc& d, int* n_partial, cudaStream_t s,
                         bool* done) {
   using Fn = int (*)(const FftAxisPlan&, PassMode, const PassDesc&, int*, cudaStream_t, bool*);
-  static const Fn kGroups[] = {fft_reg_group_0, fft_reg_group_1, fft_reg_group_2, fft_reg_group_3, fft_reg_group_4, fft_reg_group_5, fft_reg_group_6, fft_reg_group_7, fft_reg_group_8, fft_reg_group_9};
+  static const Fn kGroups[] = {fft_reg_group_0, fft_reg_group_1, fft_reg_group_2, fft_reg_group_3, fft_reg_group_4, fft_reg_group_5, fft_reg_group_6, fft_reg_group_7, fft_reg_group_8, fft_reg_group_9, fft_reg_group_10};
   *done = false;
   for (Fn f : kGroups) {
     const int st = f(a, mode, d, n_partial, s, done);

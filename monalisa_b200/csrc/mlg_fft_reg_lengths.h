@@ -72,5 +72,11 @@
   X(576, 24, 24, false) \
   X(896, 28, 32, false) \
   X(960, 32, 30, false)
+#define MLG_REG_GROUP_10(X) \
+  X(392, 28, 14, false) \
+  X(588, 28, 21, false) \
+  X(648, 24, 27, false) \
+  X(700, 28, 25, false) \
+  X(756, 28, 27, false)
 #define MLG_REG_ALL(X) \
-  MLG_REG_GROUP_0(X) MLG_REG_GROUP_1(X) MLG_REG_GROUP_2(X) MLG_REG_GROUP_3(X) MLG_REG_GROUP_4(X) MLG_REG_GROUP_5(X) MLG_REG_GROUP_6(X) MLG_REG_GROUP_7(X) MLG_REG_GROUP_8(X) MLG_REG_GROUP_9(X)
+  MLG_REG_GROUP_0(X) MLG_REG_GROUP_1(X) MLG_REG_GROUP_2(X) MLG_REG_GROUP_3(X) MLG_REG_GROUP_4(X) MLG_REG_GROUP_5(X) MLG_REG_GROUP_6(X) MLG_REG_GROUP_7(X) MLG_REG_GROUP_8(X) MLG_REG_GROUP_9(X) MLG_REG_GROUP_10(X)
