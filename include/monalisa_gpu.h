@@ -420,10 +420,10 @@ int mlg_plan_get_precision(mlg_plan_t p, int* precision);
 /* *on != 0 when a mixed solve of this plan keeps the intermediate of its
  * 3-D transforms (after the forward y pass, after the adjoint z pass) in
  * scaled FP16 inside the CG steps: MLG_PRECISION_MIXED, 3-D, a multiple of 4
- * coils, no fused adjoint gather, and TMA line passes for those shapes (bit
- * 0); bit 1 set when the forward grid is stored in scaled FP16 as well (the
- * last forward pass writes it, Gu's gathers read it: even coil count, no Gu
- * row longer than 256 entries); 0 otherwise.  No reference counterpart. */
+ * coils, no fused adjoint gather, and TMA or register line passes for those
+ * shapes (bit 0); bit 1 set when the forward grid is stored in scaled FP16 as
+ * well (the last forward pass writes it, Gu's gathers read it: even coil count,
+ * no Gu row longer than 256 entries); 0 otherwise.  No reference counterpart. */
 int mlg_plan_get_half_intermediate(mlg_plan_t p, int* on);
 
 /* Times the stages of one Shanna and one Nakatsha on the plan's stream with

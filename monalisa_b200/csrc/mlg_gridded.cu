@@ -134,17 +134,33 @@ extern "C" int mlg_gridded_tail_dev(int imDim, const int* N_u, const int* n_u, c
   cufftHandle h;
   int nn[3];
   for (int d = 0; d < imDim; ++d) nn[d] = t.N[imDim - 1 - d];
-  MLG_CUFFT(cufftPlanMany(&h, imDim, nn, nullptr, 1, (int)t.Nu, nullptr, 1, (int)t.Nu, CUFFT_C2C, nCh));
-  cufftSetStream(h, s);
-  const cufftResult r = cufftExecC2C(h, (cufftComplex*)cm.p, (cufftComplex*)cm.p, CUFFT_INVERSE);
+  // the work area comes from the stream's pool: the plan's own is a cudaMalloc and
+  // a cudaFree on every call, which wait for the device and take milliseconds
+  MLG_CUFFT(cufftCreate(&h));
+  DevBuf<char> work;
+  size_t work_bytes = 0;
+  cufftResult r = cufftSetAutoAllocation(h, 0);
+  if (r == CUFFT_SUCCESS)
+    r = cufftMakePlanMany(h, imDim, nn, nullptr, 1, (int)t.Nu, nullptr, 1, (int)t.Nu, CUFFT_C2C, nCh, &work_bytes);
+  if (r == CUFFT_SUCCESS && work_bytes > 0) {
+    const int st = work.alloc(work_bytes, s);
+    if (st != MLG_OK) {
+      cufftDestroy(h);
+      return st;
+    }
+    r = cufftSetWorkArea(h, work.p);
+  }
+  if (r == CUFFT_SUCCESS) r = cufftSetStream(h, s);
+  if (r == CUFFT_SUCCESS) r = cufftExecC2C(h, (cufftComplex*)cm.p, (cufftComplex*)cm.p, CUFFT_INVERSE);
   count_launch();
   if (r != CUFFT_SUCCESS) {
+    cudaStreamSynchronize(s);
     cufftDestroy(h);
-    return fail(MLG_ERR_CUDA, "gridded tail: cufftExecC2C failed (%d)", (int)r);
+    return fail(MLG_ERR_CUDA, "gridded tail: cuFFT failed (%d)", (int)r);
   }
   gt_tail_kernel<<<gt_grid(t.nu), kGtThreads, 0, s>>>(cm.p, t, K, (const float2*)C, (float2*)x);
   MLG_LAUNCHED();
-  // the plan's work area belongs to the calls queued on s: wait before freeing it
+  // the plan's tables belong to the calls queued on s: wait before freeing them
   const cudaError_t e = cudaStreamSynchronize(s);
   cufftDestroy(h);
   if (e != cudaSuccess) return fail(MLG_ERR_CUDA, "gridded tail failed: %s", cudaGetErrorString(e));

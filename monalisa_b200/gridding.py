@@ -19,13 +19,12 @@ def _point(a, dtype):
     return a[None, :] if a.ndim == 1 else a
 
 
-def _leight_prepare(data_n, t, Dn, N_u, dK_u):
-    """Argument preparation of bmGridder_n2u_leight.m:40-87 (single
+def _leight_points(t, Dn, N_u, dK_u):
+    """Trajectory preparation of bmGridder_n2u_leight.m:40-87 (single
     precision): grid units, Dn / prod(dK_u), samples outside the grid box
-    deleted.  Returns aR, aI [nPt][nCh], the per-axis t, Dn, nCh, nPt and the
-    three grid extents."""
+    deleted.  Returns the per-axis t, Dn, the kept samples' mask and the three
+    grid extents."""
     t = _point(t, np.float32).copy()
-    data_n = _point(data_n, np.complex64)
     Dn = np.asarray(Dn, np.float32).ravel().copy()
     imDim = t.shape[0]
     N_u = np.ravel(N_u).astype(np.float64)
@@ -37,26 +36,47 @@ def _leight_prepare(data_n, t, Dn, N_u, dK_u):
     mask = np.zeros(t.shape[1], bool)
     for i in range(imDim):
         mask |= (t[i] < 1) | (t[i] > N_u[i])
-    t, Dn, a = t[:, ~mask], Dn[~mask], data_n[:, ~mask]
+    keep = ~mask
+    tx = [np.ascontiguousarray(t[i][keep]) for i in range(imDim)] + [None] * (3 - imDim)
+    Ns = [int(N_u[i]) if i < imDim else 1 for i in range(3)]
+    return tx, np.ascontiguousarray(Dn[keep]), keep, Ns
+
+
+def _leight_prepare(data_n, t, Dn, N_u, dK_u):
+    """_leight_points and the kept samples' data: aR, aI [nPt][nCh], the
+    per-axis t, Dn, nCh, nPt and the three grid extents."""
+    data_n = _point(data_n, np.complex64)
+    tx, Dn, keep, Ns = _leight_points(t, Dn, N_u, dK_u)
+    a = data_n[:, keep]
     nCh, nPt = a.shape
     aR = np.ascontiguousarray(a.real.T, np.float32)
     aI = np.ascontiguousarray(a.imag.T, np.float32)
-    tx = [np.ascontiguousarray(t[i]) for i in range(imDim)] + [None] * (3 - imDim)
-    Ns = [int(N_u[i]) if i < imDim else 1 for i in range(3)]
-    return aR, aI, tx, np.ascontiguousarray(Dn), nCh, nPt, Ns
+    return aR, aI, tx, Dn, nCh, nPt, Ns
 
 
 def bmGridder_n2u_leight_dev(data_n, t, Dn, N_u, dK_u, kernelType=None, nWin=None, kernelParam=None):
     """The leight gridder with its output left on the device: returns CUDA
-    float32 tensors (bR, bI), each [prod(N_u)][nCh] (point layout)."""
+    float32 tensors (bR, bI), each [prod(N_u)][nCh] (point layout).  The data
+    are copied as they are (point-major complex data without a pass over them
+    on the host); samples outside the box are dropped and the parts split on
+    the device."""
     import torch
 
     kernelType, nWin, kp = kernel_defaults(kernelType, nWin, kernelParam)
-    aR, aI, tx, Dn, nCh, nPt, Ns = _leight_prepare(data_n, t, Dn, N_u, dK_u)
+    data_n = _point(data_n, np.complex64)
+    nCh, n_all = data_n.shape
+    tx, Dn, keep, Ns = _leight_points(t, Dn, N_u, dK_u)
+    if keep.size != n_all:
+        raise IndexError(f"data of {n_all} samples for a trajectory of {keep.size}")
+    nPt = Dn.size
     imDim = np.ravel(N_u).size
     dev = torch.device("cuda", torch.cuda.current_device())
     up = lambda a: torch.from_numpy(a).to(dev) if a is not None else None
-    dA, dI, dD = up(aR), up(aI), up(Dn)
+    d = up(np.require(data_n.T, requirements=["C", "W"]))
+    if nPt != n_all:
+        d = d[up(np.flatnonzero(keep))]
+    dA, dI, dD = d.real.contiguous(), d.imag.contiguous(), up(Dn)
+    del d
     dT = [up(v) for v in tx]
     nu = int(np.prod(Ns))
     bR = torch.empty((nu, nCh), dtype=torch.float32, device=dev)

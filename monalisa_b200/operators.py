@@ -215,7 +215,7 @@ class NufftPlan:
         """Whether the CG steps of a mixed solve keep the intermediate of the
         3-D transforms (after the y pass of the forward, the z pass of the
         adjoint) in scaled FP16: mixed precision on a plan whose passes support
-        it (3-D, a multiple of 4 coils, TMA line passes)."""
+        it (3-D, a multiple of 4 coils, TMA or register line passes)."""
         m = ctypes.c_int()
         N.call("mlg_plan_get_half_intermediate", self._h, ctypes.byref(m))
         return bool(m.value & 1)
@@ -411,11 +411,11 @@ def _gridded_tail(ga, gb, N_u, n_u, dK_u, nCh, C, kernelType, nWin, kp, K=None):
     N_u = _ints(N_u)
     n_u = _ints(n_u if n_u is not None else N_u)
     dev = ga.device
-    if K is None:
-        Kv = bmK(N_u, dK_u, 1, kernelType, nWin, kp)[:, 0]
+    if K is None:  # computed there (bit-identical); on the host in FP64 it took most of a small call
+        Kd = bmK_dev(N_u, dK_u, kernelType, nWin, kp)
     else:  # [prod(N_u)] or [prod(N_u), nCh] (identical columns)
         Kv = np.asarray(K, np.float32).reshape(int(np.prod(N_u)), -1, order="F")[:, 0]
-    Kd = torch.from_numpy(np.ascontiguousarray(Kv, np.float32)).to(dev)
+        Kd = torch.from_numpy(np.ascontiguousarray(Kv, np.float32)).to(dev)
     nu = int(np.prod(n_u))
     Cd = None
     if C is not None:
