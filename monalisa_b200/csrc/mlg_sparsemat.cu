@@ -775,7 +775,7 @@ static long long spmm_rows(const SpmmArgs& a) { return a.nonempty_only ? a.m->n_
 static int rows_per_block(const SpmmArgs& a) {
   const int lanes = std::max(1, point_pairs(a) ? a.nCh / 2 : a.nCh);
   const int least = std::max(1, 256 / lanes), most = std::max(1, 1024 / lanes);
-  const long long want = (spmm_rows(a) + 148 * 6 - 1) / (148 * 6);
+  const long long want = std::max<long long>(1, (spmm_rows(a) + 148 * 6 - 1) / (148 * 6));
   return (int)std::min<long long>(most, (want + least - 1) / least * least);
 }
 

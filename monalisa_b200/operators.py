@@ -412,7 +412,7 @@ def _gridded_tail(ga, gb, N_u, n_u, dK_u, nCh, C, kernelType, nWin, kp, K=None):
     n_u = _ints(n_u if n_u is not None else N_u)
     dev = ga.device
     if K is None:  # computed there (bit-identical); on the host in FP64 it took most of a small call
-        Kd = bmK_dev(N_u, dK_u, kernelType, nWin, kp)
+        Kd = bmK_dev(N_u, dK_u, kernelType, nWin, kp).to(dev)
     else:  # [prod(N_u)] or [prod(N_u), nCh] (identical columns)
         Kv = np.asarray(K, np.float32).reshape(int(np.prod(N_u)), -1, order="F")[:, 0]
         Kd = torch.from_numpy(np.ascontiguousarray(Kv, np.float32)).to(dev)

@@ -131,3 +131,28 @@ def test_gut_rows_of_every_length(nCh):
     ref = rec.plan.nakatsha(y, HY=HY, scale=3.0).cpu().numpy()
     assert rel(first, ref) <= 4e-6, rel(first, ref)
     rec.plan.close()
+
+
+@pytest.mark.parametrize("nCh", [1, 4])
+@pytest.mark.parametrize("nPt", [1, 300])
+def test_products_without_rows(nCh, nPt):
+    """All samples far outside the grid: Gu's rows and Gut's list of non-empty
+    rows are empty, both operators give zeros."""
+    import torch
+
+    import monalisa_b200 as mb
+
+    Gu, Gut = mb.bmTraj2SparseMat(np.full((2, nPt), 500.0), np.ones(nPt), [32, 32], [1, 1])
+    rng = np.random.default_rng(0)
+    C = (rng.standard_normal((256, nCh)) + 1j * rng.standard_normal((256, nCh))).astype(np.complex64)
+    rec = mb.SensaRecon(Gu, Gut, C, [16, 16])
+    y = torch.ones((rec.nPt, nCh), dtype=torch.complex64, device="cuda")
+    for mode in ("full_grid", "masked"):
+        try:
+            rec.plan.adjoint_mode = mode
+        except (mb.MonalisaError, ValueError):  # not offered for this coil count
+            continue
+        assert float(rec.plan.nakatsha(y).abs().max()) == 0
+    x = torch.ones(256, dtype=torch.complex64, device="cuda")
+    assert rec.plan.shanna(x).shape == (rec.nPt, nCh) and float(rec.plan.shanna(x).abs().max()) == 0
+    rec.plan.close()
