@@ -981,18 +981,25 @@ __device__ __forceinline__ void heavy_partial(const LeightGeom& g, const int* b,
   }
 }
 
-// Warp sum of the coil partials in a fixed butterfly order: every lane ends
-// with the totals.
-__device__ __forceinline__ void warp_sum_coils(float* ar, float* ai, float& ws) {
+// Warp sums of 2 kHeavyCoils = 32 coil partials (16 real, 16 imaginary): each
+// step of the butterfly halves the values a lane still holds, so lane l ends
+// with the total of value l after 31 shuffles (and 5 for ws, whose total every
+// lane gets); a butterfly of every value took 165 and a large share of the
+// mid cells' time.  The pairs are added as there: the same sums.  The whole call:
+// 256^3 x 16 coils 1466 -> 1448 us, 224^3 x 16 coils 960 -> 929, 64^3 x 16 252 -> 242.
+__device__ __forceinline__ float warp_sum_coils(float (&a)[2 * kHeavyCoils], float& ws, int lane) {
+  static_assert(2 * kHeavyCoils == 32, "a value per lane");
 #pragma unroll
-  for (int sh = 16; sh > 0; sh >>= 1) {
-    ws += __shfl_xor_sync(0xffffffffu, ws, sh);
+  for (int n = 16; n > 0; n >>= 1) {
+    ws += __shfl_xor_sync(0xffffffffu, ws, n);
+    const bool up = (lane & n) != 0;
 #pragma unroll
-    for (int c = 0; c < kHeavyCoils; ++c) {
-      ar[c] += __shfl_xor_sync(0xffffffffu, ar[c], sh);
-      ai[c] += __shfl_xor_sync(0xffffffffu, ai[c], sh);
+    for (int i = 0; i < n; ++i) {
+      const float keep = up ? a[i + n] : a[i], send = up ? a[i] : a[i + n];
+      a[i] = keep + __shfl_xor_sync(0xffffffffu, send, n);
     }
   }
+  return a[0];
 }
 
 // Mid cells (kHeavyIncidences < T <= kHugeIncidences, at most kMidRows
@@ -1036,19 +1043,15 @@ __global__ void __launch_bounds__(256) leight_mid_kernel(LeightGeom g, CornerGri
     const float fx = (float)(x + 1), fy = (float)(y + 1), fz = (float)(z + 1);
     for (int c0 = 0; c0 < g.nCh; c0 += kHeavyCoils) {
       const int nc = min(kHeavyCoils, g.nCh - c0);
-      float ar[kHeavyCoils], ai[kHeavyCoils], ws = 0.f;
+      float a[2 * kHeavyCoils], ws = 0.f;
 #pragma unroll
-      for (int c = 0; c < kHeavyCoils; ++c) ar[c] = ai[c] = 0.f;
-      heavy_partial<VEC4>(g, s_b[warp], s_pre[warp], T, lane, 32, rec, sidx, in, c0, nc, fx, fy, fz, ar, ai, ws);
-      warp_sum_coils(ar, ai, ws);
+      for (int c = 0; c < 2 * kHeavyCoils; ++c) a[c] = 0.f;
+      heavy_partial<VEC4>(g, s_b[warp], s_pre[warp], T, lane, 32, rec, sidx, in, c0, nc, fx, fy, fz, a, a + kHeavyCoils,
+                          ws);
+      const float sum = warp_sum_coils(a, ws, lane);
       const float inv = ws < 1e-5f ? 1.0f : __frcp_rn(ws);  // as in leight_cell_kernel
-#pragma unroll
-      for (int c = 0; c < kHeavyCoils; ++c) {
-        if (lane == c && c < nc) {
-          out.re[(long long)cell * g.nCh + c0 + c] = __fmul_rn(ar[c], inv);
-          out.im[(long long)cell * g.nCh + c0 + c] = __fmul_rn(ai[c], inv);
-        }
-      }
+      if (lane % kHeavyCoils < nc)
+        (lane < kHeavyCoils ? out.re : out.im)[(long long)cell * g.nCh + c0 + lane % kHeavyCoils] = __fmul_rn(sum, inv);
     }
   }
 }
@@ -1090,27 +1093,22 @@ __global__ void __launch_bounds__(256) leight_heavy_kernel(LeightGeom g, CornerG
     const float fx = (float)(x + 1), fy = (float)(y + 1), fz = (float)(z + 1);
     for (int c0 = 0; c0 < g.nCh; c0 += kHeavyCoils) {
       const int nc = min(kHeavyCoils, g.nCh - c0);
-      float ar[kHeavyCoils], ai[kHeavyCoils], ws = 0.f;
+      float a[2 * kHeavyCoils], ws = 0.f;
 #pragma unroll
-      for (int c = 0; c < kHeavyCoils; ++c) ar[c] = ai[c] = 0.f;
-      heavy_partial<VEC4>(g, s_b, s_pre, T, threadIdx.x, 256, rec, sidx, in, c0, nc, fx, fy, fz, ar, ai, ws);
-      warp_sum_coils(ar, ai, ws);
-      if (lane == 0) {
-        red[warp][0] = ws;
-#pragma unroll
-        for (int c = 0; c < kHeavyCoils; ++c) {
-          red[warp][1 + 2 * c] = ar[c];
-          red[warp][2 + 2 * c] = ai[c];
-        }
-      }
+      for (int c = 0; c < 2 * kHeavyCoils; ++c) a[c] = 0.f;
+      heavy_partial<VEC4>(g, s_b, s_pre, T, threadIdx.x, 256, rec, sidx, in, c0, nc, fx, fy, fz, a, a + kHeavyCoils,
+                          ws);
+      const float sum = warp_sum_coils(a, ws, lane);
+      if (lane == 0) red[warp][2 * kHeavyCoils] = ws;
+      red[warp][lane] = sum;
       __syncthreads();
       if ((int)threadIdx.x < nc) {
         const int c = threadIdx.x;
         float sw = 0.f, sr = 0.f, si = 0.f;
         for (int k = 0; k < 8; ++k) {
-          sw += red[k][0];
-          sr += red[k][1 + 2 * c];
-          si += red[k][2 + 2 * c];
+          sw += red[k][2 * kHeavyCoils];
+          sr += red[k][c];
+          si += red[k][kHeavyCoils + c];
         }
         const float inv = sw < 1e-5f ? 1.0f : __frcp_rn(sw);  // as in leight_cell_kernel
         out.re[(long long)cell * g.nCh + c0 + c] = __fmul_rn(sr, inv);
