@@ -172,15 +172,43 @@ __global__ void order_bounds_kernel(const uint32_t* __restrict__ row_ptr, const 
   }
 }
 
-// The heavy rows (ord_rows from ord_short on) cut into units of at most
+// A cudaMalloc'd table, freed unless released: the builders below assign a
+// matrix's fields once all of a group's tables stand, so that a failed
+// allocation leaves the matrix as it was and a later call builds them again.
+template <class T>
+struct DevTable {
+  T* p = nullptr;
+  ~DevTable() { cudaFree(p); }
+  int alloc(size_t n) {
+    const cudaError_t e = cudaMalloc(&p, sizeof(T) * std::max<size_t>(1, n));
+    if (e == cudaSuccess) return MLG_OK;
+    cudaGetLastError();
+    p = nullptr;
+    return fail(e == cudaErrorMemoryAllocation ? MLG_ERR_OOM : MLG_ERR_CUDA, "matrix tables: %s",
+                cudaGetErrorString(e));
+  }
+  T* release() {
+    T* q = p;
+    p = nullptr;
+    return q;
+  }
+};
+
+struct HeavyTables {
+  DevTable<int4> units;
+  DevTable<int2> multi;
+  int n_units = 0, n_multi = 0, n_multi_units = 0;
+};
+
+// The heavy rows (ordered rows from `first` on) cut into units of at most
 // kUnitLen entries, rows of several units first.
-static int csr_build_units(Csr& c, cudaStream_t s) {
-  const int nh = c.n_ord - c.ord_short;
+static int build_units(const int* ord, const uint2* bounds, int first, int n_ord, HeavyTables& t, cudaStream_t s) {
+  const int nh = n_ord - first;
   if (nh <= 0) return MLG_OK;
   std::vector<int> rows(nh);
   std::vector<uint2> be(nh);
-  MLG_CUDA(cudaMemcpyAsync(rows.data(), c.ord_rows + c.ord_short, sizeof(int) * nh, cudaMemcpyDeviceToHost, s));
-  MLG_CUDA(cudaMemcpyAsync(be.data(), c.ord_bounds + c.ord_short, sizeof(uint2) * nh, cudaMemcpyDeviceToHost, s));
+  MLG_CUDA(cudaMemcpyAsync(rows.data(), ord + first, sizeof(int) * nh, cudaMemcpyDeviceToHost, s));
+  MLG_CUDA(cudaMemcpyAsync(be.data(), bounds + first, sizeof(uint2) * nh, cudaMemcpyDeviceToHost, s));
   MLG_CUDA(cudaStreamSynchronize(s));
   std::vector<int4> units, single;
   std::vector<int2> multi;
@@ -196,14 +224,14 @@ static int csr_build_units(Csr& c, cudaStream_t s) {
                                 (int)(b + (uint32_t)((unsigned long long)n * (j + 1) / k)), (int)multi.size()));
     multi.push_back(make_int2((int)units.size() - k, k));
   }
-  c.n_multi = (int)multi.size();
-  c.n_multi_units = (int)units.size();
+  t.n_multi = (int)multi.size();
+  t.n_multi_units = (int)units.size();
   units.insert(units.end(), single.begin(), single.end());
-  c.n_units = (int)units.size();
-  MLG_CUDA(cudaMalloc(&c.heavy_units, sizeof(int4) * units.size()));
-  MLG_CUDA(cudaMalloc(&c.heavy_multi, sizeof(int2) * std::max<size_t>(1, multi.size())));
-  MLG_CUDA(cudaMemcpyAsync(c.heavy_units, units.data(), sizeof(int4) * units.size(), cudaMemcpyHostToDevice, s));
-  MLG_CUDA(cudaMemcpyAsync(c.heavy_multi, multi.data(), sizeof(int2) * multi.size(), cudaMemcpyHostToDevice, s));
+  t.n_units = (int)units.size();
+  MLG_TRY(t.units.alloc(units.size()));
+  MLG_TRY(t.multi.alloc(multi.size()));
+  MLG_CUDA(cudaMemcpyAsync(t.units.p, units.data(), sizeof(int4) * units.size(), cudaMemcpyHostToDevice, s));
+  MLG_CUDA(cudaMemcpyAsync(t.multi.p, multi.data(), sizeof(int2) * multi.size(), cudaMemcpyHostToDevice, s));
   MLG_CUDA(cudaStreamSynchronize(s));
   return MLG_OK;
 }
@@ -230,50 +258,49 @@ int csr_build_order(Csr& c, const int* N, bool nonempty, cudaStream_t s) {
   count_launch();
   int h_mid = 0;
   MLG_CUDA(cudaMemcpyAsync(&h_mid, n_mid.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  int* ord = nullptr;
-  uint2* bounds = nullptr;
-  MLG_CUDA(cudaMalloc(&ord, sizeof(int) * (size_t)std::max(1, n)));
-  if (cudaMalloc(&bounds, sizeof(uint2) * (size_t)std::max(1, n)) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(ord);
-    return fail(MLG_ERR_OOM, "row order: device allocation failed");
-  }
+  DevTable<int> ord;
+  DevTable<uint2> bounds;
+  HeavyTables heavy;
+  MLG_TRY(ord.alloc((size_t)n));
+  MLG_TRY(bounds.alloc((size_t)n));
   size_t tb = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, tb, keys.p, keys_out.p, vals.p, ord, n);
+  cub::DeviceRadixSort::SortPairs(nullptr, tb, keys.p, keys_out.p, vals.p, ord.p, n);
   DevBuf<char> tmp;
-  int st = tmp.alloc(std::max<size_t>(tb, 1), s);
-  if (st == MLG_OK && cub::DeviceRadixSort::SortPairs(tmp.p, tb, keys.p, keys_out.p, vals.p, ord, n, 0, 32, s) !=
-                          cudaSuccess)
-    st = fail(MLG_ERR_CUDA, "row order: sort failed");
-  if (st != MLG_OK) {
-    cudaFree(ord);
-    cudaFree(bounds);
-    return st;
-  }
-  order_bounds_kernel<<<g, 256, 0, s>>>(c.row_ptr, ord, n, bounds);
+  MLG_TRY(tmp.alloc(std::max<size_t>(tb, 1), s));
+  if (cub::DeviceRadixSort::SortPairs(tmp.p, tb, keys.p, keys_out.p, vals.p, ord.p, n, 0, 32, s) != cudaSuccess)
+    return fail(MLG_ERR_CUDA, "row order: sort failed");
+  order_bounds_kernel<<<g, 256, 0, s>>>(c.row_ptr, ord.p, n, bounds.p);
   count_launch();
   MLG_CUDA(cudaStreamSynchronize(s));
-  c.ord_rows = ord;
-  c.ord_bounds = bounds;
+  const int n_short = split ? n - h_mid : -1;
+  if (split) MLG_TRY(build_units(ord.p, bounds.p, n_short, n, heavy, s));
+  c.ord_rows = ord.release();
+  c.ord_bounds = bounds.release();
   c.n_ord = n;
   c.ord_nonempty = nonempty;
-  c.ord_short = split ? n - h_mid : -1;
-  return split ? csr_build_units(c, s) : MLG_OK;
+  c.ord_short = n_short;
+  c.heavy_units = heavy.units.release();
+  c.heavy_multi = heavy.multi.release();
+  c.n_units = heavy.n_units;
+  c.n_multi = heavy.n_multi;
+  c.n_multi_units = heavy.n_multi_units;
+  return MLG_OK;
 }
 
 int csr_build_nonempty(Csr& c, cudaStream_t s) {
   if (c.nz_mask) return MLG_OK;
   const int nw = (c.l_size + 31) / 32;
-  int *cnt = nullptr, *off = nullptr;
-  MLG_CUDA(cudaMalloc(&c.nz_mask, sizeof(uint32_t) * (size_t)std::max(1, nw)));
-  MLG_CUDA(cudaMalloc(&cnt, sizeof(int) * (size_t)(nw + 1)));
-  MLG_CUDA(cudaMalloc(&off, sizeof(int) * (size_t)(nw + 1)));
+  DevTable<uint32_t> mask;
+  DevTable<int> cnt, off, rows;
+  MLG_TRY(mask.alloc((size_t)nw));
+  MLG_TRY(cnt.alloc((size_t)(nw + 1)));
+  MLG_TRY(off.alloc((size_t)(nw + 1)));
   const int g = std::max(1, std::min(4096, (nw + 255) / 256));
-  nz_mask_kernel<<<g, 256, 0, s>>>(c.row_ptr, c.l_size, c.nz_mask, cnt);
+  nz_mask_kernel<<<g, 256, 0, s>>>(c.row_ptr, c.l_size, mask.p, cnt.p);
   count_launch();
   // exclusive scan of the word counts on the host (nw is small: l_size/32)
   std::vector<int> h(nw + 1, 0);
-  MLG_CUDA(cudaMemcpyAsync(h.data(), cnt, sizeof(int) * nw, cudaMemcpyDeviceToHost, s));
+  MLG_CUDA(cudaMemcpyAsync(h.data(), cnt.p, sizeof(int) * nw, cudaMemcpyDeviceToHost, s));
   MLG_CUDA(cudaStreamSynchronize(s));
   int run = 0;
   for (int w = 0; w < nw; ++w) {
@@ -282,14 +309,14 @@ int csr_build_nonempty(Csr& c, cudaStream_t s) {
     run += v;
   }
   h[nw] = run;
-  c.n_nonempty = run;
-  MLG_CUDA(cudaMemcpyAsync(off, h.data(), sizeof(int) * (nw + 1), cudaMemcpyHostToDevice, s));
-  MLG_CUDA(cudaMalloc(&c.nz_rows, sizeof(int) * (size_t)std::max(1, run)));
-  nz_rows_kernel<<<g, 256, 0, s>>>(c.nz_mask, off, nw, c.nz_rows);
+  MLG_TRY(rows.alloc((size_t)run));
+  MLG_CUDA(cudaMemcpyAsync(off.p, h.data(), sizeof(int) * (nw + 1), cudaMemcpyHostToDevice, s));
+  nz_rows_kernel<<<g, 256, 0, s>>>(mask.p, off.p, nw, rows.p);
   count_launch();
   MLG_CUDA(cudaStreamSynchronize(s));
-  cudaFree(cnt);
-  cudaFree(off);
+  c.nz_mask = mask.release();
+  c.nz_rows = rows.release();
+  c.n_nonempty = run;
   return MLG_OK;
 }
 

@@ -853,6 +853,7 @@ int spmm(const SpmmArgs& a, cudaStream_t s) {
   const int grid_short = a.long_only ? 0 : grid_all;
   p.partial_long_offset = grid_all;
   MLG_CHECK(m.n_long == 0 || m.n_seg > 0, "long rows without segment tables");
+  MLG_CHECK(m.n_units == 0 || (m.heavy_units && m.heavy_multi), "heavy rows without unit tables");
   DevBuf<float> own;
   float* scratch = a.seg_scratch;
   if ((m.n_long > 0 || m.n_multi_units > 0) && !scratch) {
