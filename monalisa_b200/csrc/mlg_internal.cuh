@@ -113,6 +113,33 @@ struct DevBuf {
   }
 };
 
+// A caller's operand of n complex values.  The kernels of even coil counts move
+// coil pairs, 16 bytes at a time: where the pointer is only 8-byte aligned (an
+// odd offset into a larger buffer) they work on an aligned copy instead, made
+// by in() and, for results, written back by finish().
+struct PairOperand {
+  float2* p = nullptr;
+  void* user = nullptr;
+  DevBuf<float2> copy;
+  int out(const void* ptr, size_t n, bool pairs, cudaStream_t s) {
+    user = const_cast<void*>(ptr);
+    p = static_cast<float2*>(user);
+    if (!pairs || n == 0 || reinterpret_cast<uintptr_t>(ptr) % 16 == 0) return MLG_OK;
+    MLG_TRY(copy.alloc(n, s));
+    p = copy.p;
+    return MLG_OK;
+  }
+  int in(const void* ptr, size_t n, bool pairs, cudaStream_t s) {
+    MLG_TRY(out(ptr, n, pairs, s));
+    if (copy.p) MLG_CUDA(cudaMemcpyAsync(copy.p, ptr, sizeof(float2) * n, cudaMemcpyDeviceToDevice, s));
+    return MLG_OK;
+  }
+  int finish() {
+    if (copy.p) MLG_CUDA(cudaMemcpyAsync(user, copy.p, sizeof(float2) * copy.n, cudaMemcpyDeviceToDevice, copy.s));
+    return MLG_OK;
+  }
+};
+
 // ---- device CSR -----------------------------------------------------------
 // Absolute-index CSR with a dense row pointer over all l_size rows (rows the
 // jump format squeezes out are empty).  Long rows (more than kLongRow

@@ -784,7 +784,12 @@ int mlg_shanna_dev(mlg_plan_t p, const void* x, int x_per_coil, void* y, void* s
   MLG_CHECK(p->Gu, "plan has no Gu");
   MLG_CUDA(cudaSetDevice(p->device));
   StreamJoin j(p, (cudaStream_t)stream);
-  return shanna_run(p, (const float2*)x, x_per_coil != 0, (float2*)y, nullptr, nullptr, nullptr, p->stream);
+  const bool pairs = p->nCh % 2 == 0;
+  PairOperand xi, yo;
+  MLG_TRY(xi.in(x, (size_t)p->nu_tot * (x_per_coil ? p->nCh : 1), pairs && x_per_coil, p->stream));
+  MLG_TRY(yo.out(y, (size_t)p->nPt * p->nCh, pairs, p->stream));
+  MLG_TRY(shanna_run(p, xi.p, x_per_coil != 0, yo.p, nullptr, nullptr, nullptr, p->stream));
+  return yo.finish();
 }
 
 int mlg_nakatsha_dev(mlg_plan_t p, const void* y, const float* HY, float scale, void* x, void* stream) {
@@ -792,7 +797,9 @@ int mlg_nakatsha_dev(mlg_plan_t p, const void* y, const float* HY, float scale, 
   MLG_CHECK(p->Gut, "plan has no Gut");
   MLG_CUDA(cudaSetDevice(p->device));
   StreamJoin j(p, (cudaStream_t)stream);
-  return nakatsha_run(p, (const float2*)y, HY, scale, (float2*)x, nullptr, nullptr, p->stream);
+  PairOperand yi;
+  MLG_TRY(yi.in(y, (size_t)p->nPt * p->nCh, p->nCh % 2 == 0, p->stream));
+  return nakatsha_run(p, yi.p, HY, scale, (float2*)x, nullptr, nullptr, p->stream);
 }
 
 // Stateless host-buffer operators (drop-ins for the CUFFT MEX files).

@@ -1175,15 +1175,19 @@ int mlg_matrix_download(mlg_matrix_t m, int* r_jump, int* r_nJump, float* m_val,
 int mlg_matrix_spmm_dev(mlg_matrix_t m, const void* v, int nVec, void* w, void* stream) {
   MLG_CHECK(m && v && w && nVec >= 1, "invalid argument");
   MLG_CUDA(cudaSetDevice(m->device));
+  PairOperand vi, wo;
+  MLG_TRY(vi.in(v, (size_t)m->csr.r_size * nVec, nVec % 2 == 0, (cudaStream_t)stream));
+  MLG_TRY(wo.out(w, (size_t)m->csr.l_size * nVec, nVec % 2 == 0, (cudaStream_t)stream));
   SpmmArgs a;
   a.m = &m->csr;
   a.nCh = nVec;
   a.in.layout = a.out.layout = Layout::kPointC64;
-  a.in.a = const_cast<void*>(v);
+  a.in.a = vi.p;
   a.in.rows = m->csr.r_size;
-  a.out.a = w;
+  a.out.a = wo.p;
   a.out.rows = m->csr.l_size;
-  return spmm(a, (cudaStream_t)stream);
+  MLG_TRY(spmm(a, (cudaStream_t)stream));
+  return wo.finish();
 }
 
 }  // extern "C"
