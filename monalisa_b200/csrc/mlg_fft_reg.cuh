@@ -295,20 +295,18 @@ __device__ __forceinline__ void reg_load(const float2* base, unsigned off, float
   }
 }
 
+// The same of FP16 rows, unconverted: a row's conversion under the condition of
+// its load waited for that load before the next went out (mixed precision, 192^3 x
+// 16 coils: inverse y pass 180 -> 121 us; 120 stored rows 243 -> 168, forward z 261
+// -> 206).
 template <int VEC>
-__device__ __forceinline__ void reg_load(const __half2* base, unsigned off, float hs, float2* a) {
-  unsigned q[VEC];
+__device__ __forceinline__ void reg_load(const __half2* base, unsigned off, unsigned* a) {
   if constexpr (VEC == 2) {
     const uint2 w = __ldcg(reinterpret_cast<const uint2*>(reg_at(base, off)));
-    q[0] = w.x;
-    q[1] = w.y;
+    a[0] = w.x;
+    a[1] = w.y;
   } else {
-    q[0] = __ldcg(reinterpret_cast<const unsigned*>(reg_at(base, off)));
-  }
-#pragma unroll
-  for (int v = 0; v < VEC; ++v) {
-    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&q[v]));
-    a[v] = make_float2(h.x * hs, h.y * hs);
+    a[0] = __ldcg(reinterpret_cast<const unsigned*>(reg_at(base, off)));
   }
 }
 
@@ -357,14 +355,20 @@ __device__ __forceinline__ void reg_load_rows(float2 (&r)[VEC][N1], const RegPas
   };
   if (half) {
     const __half2* base = reinterpret_cast<const __half2*>(in) + in0;
+    unsigned w[N1][VEC];
 #pragma unroll
     for (int n1 = 0; n1 < N1; ++n1) {
-      float2 q[VEC];
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) q[v] = make_float2(0.f, 0.f);
-      if (want(n1)) reg_load<VEC>(base + (long long)(n1 * N2) * a.in_row, off, hs, q);
+      for (int v = 0; v < VEC; ++v) w[n1][v] = 0u;
+      if (want(n1)) reg_load<VEC>(base + (long long)(n1 * N2) * a.in_row, off, w[n1]);
+    }
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) r[v][n1] = q[v];
+    for (int n1 = 0; n1 < N1; ++n1) {
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) {
+        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&w[n1][v]));
+        r[v][n1] = want(n1) ? make_float2(h.x * hs, h.y * hs) : make_float2(0.f, 0.f);
+      }
     }
   } else {
     const float2* base = reinterpret_cast<const float2*>(in) + in0;
@@ -487,8 +491,11 @@ __global__ void __launch_bounds__(reg_threads(N1, N2, COLS, VEC),
 
 // ---- forward x pass: x .* KFC, modulation, zero-fill, transform ---------------------
 // One coil per thread (two measured slower: 158 against 142 us at 256-point
-// lines of 16 coils, 69 against 60 us at 192 x 12).  TB: launch bound,
-// reg_x_bound for up to 16 coils, 1024 beyond.
+// lines of 16 coils, 69 against 60 us at 192 x 12).  Without HALF the rows' loads
+// go out eight at a time, conditions on the loads alone: with a row's product
+// under its condition each row waited for its own loads (oversampling 1.6, 256-point
+// lines of 16 coils 429 -> 290 us, 128 x 32 coils 180 -> 99, 192 x 12 167 -> 115).
+// TB: launch bound, reg_x_bound for up to 16 coils, 1024 beyond.
 constexpr int reg_x_bound(int N1, int N2) { return reg_groups(N1, N2) <= 16 ? 256 : 512; }
 
 template <int N1, int N2, bool HALF, int TB>
@@ -509,16 +516,31 @@ __global__ void __launch_bounds__(TB, reg_min_blocks(N1, N2, TB))
     if (live && g < N2) {
       const int par = (a.par0 + line % a.ny + line / a.ny) & 1;
       const long long m0 = (long long)line * a.in_len + g - a.in_lo;
+      const uint32_t word = HALF ? 0u : reg_range_word<N2>(g, a.in_lo, a.in_len);
+      constexpr int LO = HALF ? N1 / 4 : 0, HI = HALF ? 3 * N1 / 4 : N1, U = HALF ? HI - LO : 8;
       float2 r[1][N1];
 #pragma unroll
-      for (int n1 = 0; n1 < N1; ++n1) {
-        r[0][n1] = make_float2(0.f, 0.f);
-        const int n = n1 * N2 + g;
-        if (HALF ? n1 >= N1 / 4 && n1 < 3 * N1 / 4 : n >= a.in_lo && n < a.in_lo + a.in_len) {
-          const long long m = m0 + n1 * N2;
-          const float2 xv = __ldg(a.img + (a.img_per_coil ? m * C + c : m));
-          const float2 p = cmulf_rn(xv, __ldg(a.kfc + m * C + c));
-          r[0][n1] = ((n + par) & 1) ? make_float2(-p.x, -p.y) : p;
+      for (int n1 = 0; n1 < N1; ++n1) r[0][n1] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int b0 = LO; b0 < HI; b0 += U) {
+        float2 xv[U], kv[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          const int n1 = b0 + q;
+          xv[q] = kv[q] = make_float2(0.f, 0.f);
+          if (n1 < HI && (HALF || (word & (1u << n1)))) {
+            const long long m = m0 + n1 * N2;
+            xv[q] = __ldg(a.img + (a.img_per_coil ? m * C + c : m));
+            kv[q] = __ldg(a.kfc + m * C + c);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          const int n1 = b0 + q;
+          if (n1 < HI) {
+            const float2 p = cmulf_rn(xv[q], kv[q]);
+            r[0][n1] = ((n1 * N2 + g + par) & 1) ? make_float2(-p.x, -p.y) : p;
+          }
         }
       }
       reg_step_a<N1, -1, HALF, 1>(r, T, g, s, S1, C);
@@ -544,7 +566,9 @@ __global__ void __launch_bounds__(TB, reg_min_blocks(N1, N2, TB))
 // takes the L1 space the row loads need).  The products (VEC == 2: summed over the thread's coil pair) leave step C for
 // a shared-memory area of their own ([pixel][C / VEC], an odd row length: no
 // bank conflicts) and a thread per pixel sums them in four interleaved sums;
-// |x|^2 partial sums in FP64 per CTA.
+// |x|^2 partial sums in FP64 per CTA.  The coil maps' rows without HALF: four
+// loads at a time, as in the forward pass (oversampling 1.6, 256 x 16 coils 395 ->
+// 283 us, 128 x 8 58 -> 43).
 template <int N1, int N2, bool HALF, int VEC, int TB>
 __global__ void __launch_bounds__(TB, reg_min_blocks(N1, N2, TB, VEC))
     reg_nak_kernel(RegPass a, const float2* __restrict__ tw) {
@@ -582,17 +606,36 @@ __global__ void __launch_bounds__(TB, reg_min_blocks(N1, N2, TB, VEC))
       const int par = (a.par0 + line % a.ny + line / a.ny) & 1;
       const float2* kf = a.kfc + ((long long)line * a.out_len + g - a.out_lo) * C + c;
       float2* o = prod + (l * a.out_len + g - a.out_lo) * CP + c / VEC;
+      const uint32_t word = HALF ? 0u : reg_range_word<N1>(g, a.out_lo, a.out_len);
+      constexpr int LO = HALF ? N2 / 4 : 0, HI = HALF ? 3 * N2 / 4 : N2, U = HALF ? HI - LO : 4;
 #pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) {
-        const int k = g + N1 * k2;
-        if (HALF ? k2 >= N2 / 4 && k2 < 3 * N2 / 4 : k >= a.out_lo && k < a.out_lo + a.out_len) {
-          const float sg = ((k + par) & 1) ? -a.sfac : a.sfac;
-          if constexpr (VEC == 2) {
-            const float4 kv = __ldcs(reinterpret_cast<const float4*>(kf + N1 * k2 * C));
-            o[N1 * k2 * CP] = nak_pair_term(make_float4(r[0][k2].x, r[0][k2].y, r[1][k2].x, r[1][k2].y), kv, sg);
-          } else {
-            const float2 v = r[0][k2];
-            o[N1 * k2 * CP] = cmulf_rn(make_float2(__fmul_rn(v.x, sg), __fmul_rn(v.y, sg)), __ldcs(kf + N1 * k2 * C));
+      for (int b0 = LO; b0 < HI; b0 += U) {
+        float2 kv[U][VEC];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          const int k2 = b0 + q;
+          if (k2 < HI && (HALF || (word & (1u << k2)))) {
+            if constexpr (VEC == 2) {
+              const float4 v = __ldcs(reinterpret_cast<const float4*>(kf + N1 * k2 * C));
+              kv[q][0] = make_float2(v.x, v.y);
+              kv[q][1] = make_float2(v.z, v.w);
+            } else {
+              kv[q][0] = __ldcs(kf + N1 * k2 * C);
+            }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          const int k2 = b0 + q, k = g + N1 * k2;
+          if (k2 < HI && (HALF || (word & (1u << k2)))) {
+            const float sg = ((k + par) & 1) ? -a.sfac : a.sfac;
+            if constexpr (VEC == 2) {
+              o[N1 * k2 * CP] = nak_pair_term(make_float4(r[0][k2].x, r[0][k2].y, r[1][k2].x, r[1][k2].y),
+                                              make_float4(kv[q][0].x, kv[q][0].y, kv[q][1].x, kv[q][1].y), sg);
+            } else {
+              const float2 v = r[0][k2];
+              o[N1 * k2 * CP] = cmulf_rn(make_float2(__fmul_rn(v.x, sg), __fmul_rn(v.y, sg)), kv[q][0]);
+            }
           }
         }
       }
