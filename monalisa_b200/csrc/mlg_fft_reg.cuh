@@ -355,19 +355,22 @@ __device__ __forceinline__ void reg_load_rows(float2 (&r)[VEC][N1], const RegPas
   };
   if (half) {
     const __half2* base = reinterpret_cast<const __half2*>(in) + in0;
-    unsigned w[N1][VEC];
 #pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
+    for (int n1 = 0; n1 < N1; ++n1) {  // (a row's bits wait in the register of its real part)
+      unsigned w[VEC];
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) w[n1][v] = 0u;
-      if (want(n1)) reg_load<VEC>(base + (long long)(n1 * N2) * a.in_row, off, w[n1]);
+      for (int v = 0; v < VEC; ++v) w[v] = 0u;
+      if (want(n1)) reg_load<VEC>(base + (long long)(n1 * N2) * a.in_row, off, w);
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) r[v][n1].x = __uint_as_float(w[v]);
     }
 #pragma unroll
     for (int n1 = 0; n1 < N1; ++n1) {
 #pragma unroll
       for (int v = 0; v < VEC; ++v) {
-        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&w[n1][v]));
-        r[v][n1] = want(n1) ? make_float2(h.x * hs, h.y * hs) : make_float2(0.f, 0.f);
+        const unsigned w = __float_as_uint(r[v][n1].x);
+        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&w));
+        r[v][n1] = make_float2(h.x * hs, h.y * hs);  // (rows that are not stored: zeros)
       }
     }
   } else {
@@ -417,10 +420,10 @@ __device__ __forceinline__ void reg_store_rows(const float2 (&r)[VEC][N2], const
 
 // Resident threads per SM asked of the register allocator: 64 registers a
 // thread for one column of up to 16-point sub-transforms, 128 for two columns
-// or up to 32 points.
+// (96 of up to 8 points) or up to 32 points.
 constexpr int reg_min_blocks(int N1, int N2, int nt, int vec = 1) {
   const int g = reg_groups(N1, N2);
-  const int thr = vec == 2 ? 512 : (g <= 16 ? 1024 : (g <= 20 ? 768 : 512));
+  const int thr = vec == 2 ? (g <= 8 ? 640 : 512) : (g <= 16 ? 1024 : (g <= 20 ? 768 : 512));
   return thr / nt < 1 ? 1 : thr / nt;
 }
 constexpr int reg_threads(int N1, int N2, int cols, int vec) { return cols / vec * reg_groups(N1, N2); }
