@@ -190,13 +190,47 @@ static int fft_reg_pass(const FftAxisPlan& a, PassMode mode, const PassDesc& d, 
   return MLG_OK;
 }
 
+// Passes of 96- to 192-point axes that the shared-memory kernels run faster than
+// the register ones: their bundles are whole cells of 24 or 32 coils or the
+// caches hold what the column pairs re-read.  us, register / shared, forward
+// unless marked inv, over 3-D grids (image length in brackets):
+//   unmasked y passes of at least 14 M values in and out: 128 [64] x 16 coils
+//     52 / 49, 128 [80] x 8 36 / 33, x 16 69 / 60, x 32 130 / 103, 192 [96] x 12
+//     108 / 100, [120] x 16 188 / 177 (below: 128 [64] x 8 24 / 28, 96 [48] x 16
+//     22 / 23); exact halves at 192 with 8 or 16 coils 75 / 77, 141 / 144; inv to
+//     128 points and outside the exact half, 128 [80] x 16 62 / 56, at 32 coils
+//     anywhere, 128 [64] 82 / 72 (192 [120] x 24 243 / 260, 96 [48] x 24 30 / 32);
+//   masked passes at 32 coils: 96 [48] 64 / 56, 128 [80] 127 / 110, inv 133 / 115
+//     (inv 96 [48] 48 / 58, 192 300 / 380; 24 coils 96 [60] 56 / 56, 128 89 / 110);
+//   x passes at 32 coils 128 [64] 55 / 47, [80] 99 / 70, at 24 [80] 86 / 72 (24
+//     coils exact half 47 / 50, 16 coils 49 / 49);
+//   inv x passes with pipelined kernels to 128 points outside the exact half: 96
+//     [60] x 16 42 / 30, 128 [80] x 8 44 / 33 (192 [120] x 8 80 / 98, 12 coils 71 /
+//     126, exact half 17 / 22).
+// 64 points: 32 coils 15 / 18 at the most even; 256: 16 coils 284 / 315.  2-D
+// passes have too few lines: 128 [80] x 16 coils 10 / 10 to 384 [240] x 16 15 / 15.
+static bool shared_pass_faster(const FftAxisPlan& a, PassMode mode, const PassDesc& d) {
+  const int N = a.N, C = d.C, u = d.ax == 0 ? 1 : 0, v = d.ax == 2 ? 1 : 2;
+  const long long lines = (long long)d.dims[u] * d.dims[v];
+  if (!a.fast || N < 96 || N > 192 || lines < 2048 || d.tma_slots < 2 || !tma_passes_enabled()) return false;
+  const bool fwd = d.dir < 0;
+  const bool half = fwd ? d.in_lo == N / 4 && d.in_len == N / 2 : d.out_lo == N / 4 && d.out_len == N / 2;
+  if (mode == PassMode::kShannaIn) return C == 32 || (C == 24 && !half);
+  if (mode == PassMode::kNakatshaOut) return !half && N <= 128 && (C == 4 || C == 8 || C == 16);
+  if (fwd ? d.out_tmask != nullptr : d.in_mask != nullptr) return C == 32 && N <= 128 && (fwd || !half);
+  if ((C != 8 && C != 12 && C != 16 && C != 24 && C != 32) || lines * (d.in_len + d.out_len) * C < 14000000)
+    return false;
+  if (fwd) return !half || N <= 128 || C == 12 || C >= 24;
+  return N <= 128 && (!half || C == 32);
+}
+
 int fft_pass(const FftAxisPlan& a, PassMode mode, const PassDesc& d, int* n_partial, cudaStream_t s) {
   MLG_CHECK(a.N >= 1 && a.tw, "FFT axis not initialised");
   MLG_CHECK(d.C >= 1, "C must be >= 1");
   const int L = lines_per_cta(a, d.C, mode);
   MLG_CHECK((size_t)a.N * L * d.C * sizeof(float2) <= 200 * 1024,
             "FFT line of %d points x %d coils exceeds shared memory", a.N, d.C);
-  if (d.reg && !d.dry && a.rA > 0 && mode != PassMode::kGutIn) {
+  if (d.reg && !d.dry && a.rA > 0 && mode != PassMode::kGutIn && !shared_pass_faster(a, mode, d)) {
     bool done = false;
     if (n_partial) *n_partial = 0;
     MLG_TRY(fft_reg_pass(a, mode, d, n_partial, s, &done));
