@@ -676,26 +676,32 @@ __global__ void __launch_bounds__(TB, reg_min_blocks(N1, N2, TB, VEC))
 constexpr int kRegMaxBlocks = 2048;  // CTAs of a register pass (partial-sum slots)
 constexpr size_t kRegSmemCap = 200 * 1024;
 
-// Grid of a persistent kernel: resident CTAs per SM (per kernel, shared
-// memory and CTA size; kept per host thread) x SMs, at most `work`.
-template <class K>
-static int reg_grid(K kern, int threads, size_t smem, int work, int* grid) {
+// Launches a persistent kernel over `work` bundles: at most the resident CTAs of
+// the GPU.  What depends on the kernel, the CTA and the device alone is kept per
+// host thread and kernel -- KERN is a template argument, every register kernel has
+// the same pointer type: a cache by type was refilled (three runtime calls) on
+// nearly every pass.
+template <auto KERN>
+static int reg_launch(const RegPass& p, const float2* tw, int threads, size_t smem, int* grid, cudaStream_t s) {
   thread_local int per_sm = 0, sms = 0, t_threads = 0, t_dev = -1;
   thread_local size_t t_smem = 0;
-  thread_local K t_kern = nullptr;
   int dev = 0;
   MLG_CUDA(cudaGetDevice(&dev));
-  if (per_sm == 0 || t_smem != smem || t_threads != threads || t_dev != dev || t_kern != kern) {
-    MLG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRegSmemCap));
-    MLG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MLG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+  if (per_sm == 0 || t_smem != smem || t_threads != threads || t_dev != dev) {
+    if (t_dev != dev) {
+      MLG_CUDA(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRegSmemCap));
+      MLG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    }
+    per_sm = 0;
+    MLG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERN, threads, smem));
     per_sm = std::max(1, per_sm);
     t_smem = smem;
     t_threads = threads;
     t_dev = dev;
-    t_kern = kern;
   }
-  *grid = std::max(1, std::min(std::min(work, per_sm * sms), kRegMaxBlocks));
+  *grid = std::max(1, std::min(std::min(p.nbundles, per_sm * sms), kRegMaxBlocks));
+  KERN<<<*grid, threads, smem, s>>>(p, tw);
+  MLG_LAUNCHED();
   return MLG_OK;
 }
 
@@ -706,10 +712,7 @@ static int reg_plain_launch(RegPass& p, const float2* tw, cudaStream_t s) {
   p.nb_u = (p.Q + COLS - 1) / COLS;
   p.nbundles = p.nb_u * p.planes;
   int grid = 1;
-  MLG_TRY(reg_grid(reg_plain_kernel<N1, N2, DIR, COLS, VEC, HALF>, NT, smem, p.nbundles, &grid));
-  reg_plain_kernel<N1, N2, DIR, COLS, VEC, HALF><<<grid, NT, smem, s>>>(p, tw);
-  MLG_LAUNCHED();
-  return MLG_OK;
+  return reg_launch<reg_plain_kernel<N1, N2, DIR, COLS, VEC, HALF>>(p, tw, NT, smem, &grid, s);
 }
 
 // The geometry of a y or z pass; false where the register kernels do not
@@ -824,16 +827,14 @@ static int reg_shanna_pass(const PassDesc& d, const float2* tw, cudaStream_t s, 
   size_t smem = 0;
   if (!reg_x_shape(N1, N2, 1, p, 0, false, &threads, &smem)) return MLG_OK;
   constexpr int TB = reg_x_bound(N1, N2);
-  auto kern = threads <= TB ? reg_shanna_kernel<N1, N2, false, TB> : reg_shanna_kernel<N1, N2, false, 1024>;
+  *done = true;
   if constexpr (MAIN) {
     if (d.in_lo == N / 4 && d.in_len == N / 2)
-      kern = threads <= TB ? reg_shanna_kernel<N1, N2, true, TB> : reg_shanna_kernel<N1, N2, true, 1024>;
+      return threads <= TB ? reg_launch<reg_shanna_kernel<N1, N2, true, TB>>(p, tw, threads, smem, &grid, s)
+                           : reg_launch<reg_shanna_kernel<N1, N2, true, 1024>>(p, tw, threads, smem, &grid, s);
   }
-  MLG_TRY(reg_grid(kern, threads, smem, p.nbundles, &grid));
-  kern<<<grid, threads, smem, s>>>(p, tw);
-  MLG_LAUNCHED();
-  *done = true;
-  return MLG_OK;
+  return threads <= TB ? reg_launch<reg_shanna_kernel<N1, N2, false, TB>>(p, tw, threads, smem, &grid, s)
+                       : reg_launch<reg_shanna_kernel<N1, N2, false, 1024>>(p, tw, threads, smem, &grid, s);
 }
 
 template <int N1, int N2, bool MAIN>
@@ -862,24 +863,36 @@ static int reg_nak_pass(const PassDesc& d, const float2* tw, int* n_partial, cud
   const int vec = kPairs && d.C % 2 == 0 ? 2 : 1;
   if (!reg_x_shape(N1, N2, vec, p, d.out_len, true, &threads, &smem)) return MLG_OK;
   constexpr int TB = reg_x_bound(N1, N2);
-  auto kern = threads <= TB ? reg_nak_kernel<N1, N2, false, 1, TB> : reg_nak_kernel<N1, N2, false, 1, 1024>;
+  if (threads > (vec == 2 ? 512 : 1024)) return MLG_OK;
+  *done = true;
+  auto run = [&](auto half, auto v) {
+    constexpr bool H = decltype(half)::value;
+    constexpr int V = decltype(v)::value;
+    return threads <= TB
+               ? reg_launch<reg_nak_kernel<N1, N2, H, V, TB>>(p, tw, threads, smem, &grid, s)
+               : reg_launch<reg_nak_kernel<N1, N2, H, V, V == 2 ? 512 : 1024>>(p, tw, threads, smem, &grid, s);
+  };
+  using std::bool_constant;
+  using std::integral_constant;
+  int st;
   if constexpr (MAIN) {
     const bool half = d.out_lo == N / 4 && d.out_len == N / 2;
-    if (half) kern = threads <= TB ? reg_nak_kernel<N1, N2, true, 1, TB> : reg_nak_kernel<N1, N2, true, 1, 1024>;
     if constexpr (kPairs) {
-      if (vec == 2 && half)
-        kern = threads <= TB ? reg_nak_kernel<N1, N2, true, 2, TB> : reg_nak_kernel<N1, N2, true, 2, 512>;
-      else if (vec == 2)
-        kern = threads <= TB ? reg_nak_kernel<N1, N2, false, 2, TB> : reg_nak_kernel<N1, N2, false, 2, 512>;
+      if (vec == 2)
+        st = half ? run(bool_constant<true>(), integral_constant<int, 2>())
+                  : run(bool_constant<false>(), integral_constant<int, 2>());
+      else
+        st = half ? run(bool_constant<true>(), integral_constant<int, 1>())
+                  : run(bool_constant<false>(), integral_constant<int, 1>());
+    } else {
+      st = half ? run(bool_constant<true>(), integral_constant<int, 1>())
+                : run(bool_constant<false>(), integral_constant<int, 1>());
     }
+  } else {
+    st = run(bool_constant<false>(), integral_constant<int, 1>());
   }
-  if (threads > (vec == 2 ? 512 : 1024)) return MLG_OK;
-  MLG_TRY(reg_grid(kern, threads, smem, p.nbundles, &grid));
-  kern<<<grid, threads, smem, s>>>(p, tw);
-  MLG_LAUNCHED();
   if (n_partial) *n_partial = d.partial ? grid : 0;
-  *done = true;
-  return MLG_OK;
+  return st;
 }
 
 // Pass `mode` over an axis of length A * B (A a multiple of 4): the forward
