@@ -351,12 +351,12 @@ int mlg_idf(int imDim, const int* N_u, const float* dK_u, int nCol,
  * product: MLG_ADJ_FULL_GRID writes every grid cell and streams the grid;
  * MLG_ADJ_FUSED gathers the Gut rows inside the pass (2-D/3-D);
  * MLG_ADJ_MASKED writes only the non-empty Gut rows and reads a cell only if
- * its occupancy bit is set (even nCh).  All give the same values up to
- * floating-point summation order of the long rows.  Tuning API; no reference
- * counterpart. */
-/* An odd coil count (2-D, 3-D; at most 32) with register passes
- * (mlg_plan_set_register_passes) runs the masked strategy's kernels, a coil
- * per thread, whichever strategy is set. */
+ * its occupancy bit is set (even nCh; odd nCh up to 32 in 2-D and 3-D where the
+ * last axis has register passes, mlg_plan_set_register_passes, and they are on:
+ * where they are turned off, such a plan runs, and mlg_plan_get_adjoint reports,
+ * the fused strategy, or the full grid in reduced precision).  All give the same values up to
+ * floating-point summation order of the long rows.  Plans start on the masked
+ * strategy where they have it.  Tuning API; no reference counterpart. */
 #define MLG_ADJ_FULL_GRID 0
 #define MLG_ADJ_FUSED 1
 #define MLG_ADJ_MASKED 2

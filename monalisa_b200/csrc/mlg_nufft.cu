@@ -137,10 +137,14 @@ static int forward_pass(mlg_plan_s* p, int ax, const float2* x, bool x_per_coil,
 // reads the grid written by the Gut product.
 enum : int { kAdjFullGrid = 0, kAdjFused = 1, kAdjMasked = 2 };
 
-// the strategy an adjoint runs (see odd_masked)
-static int run_mode(const mlg_plan_s* p) { return p->odd_masked && p->reg_passes ? (int)kAdjMasked : p->adjoint_mode; }
+// the strategy an adjoint runs: the plan's, but the masked one of odd coil counts
+// exists with register passes only
+int adjoint_run_mode(const mlg_plan_s* p) {
+  if (p->adjoint_mode != kAdjMasked || p->nCh % 2 == 0 || p->reg_passes) return p->adjoint_mode;
+  return p->precision == MLG_PRECISION_FP32 ? kAdjFused : kAdjFullGrid;
+}
 
-static bool fused_gut(const mlg_plan_s* p) { return run_mode(p) == kAdjFused; }
+static bool fused_gut(const mlg_plan_s* p) { return adjoint_run_mode(p) == kAdjFused; }
 
 // adjoint variants a plan can run
 bool adjoint_mode_valid(const mlg_plan_s* p, int mode) {
@@ -148,8 +152,9 @@ bool adjoint_mode_valid(const mlg_plan_s* p, int mode) {
   // the fused gather reads FP32 k-space and FP32 values inside the FFT pass:
   // FP32 plans only
   if (mode == kAdjFused) return p->imDim >= 2 && p->precision == MLG_PRECISION_FP32;
+  if (mode == kAdjMasked && p->nCh % 2) return p->odd_masked && p->reg_passes;
   if (mode == kAdjMasked)
-    return (p->nCh % 2) == 0 && p->Gut_s.nz_mask != nullptr && p->Gut_s.ord_rows != nullptr && p->Gut_s.ord_nonempty;
+    return p->Gut_s.nz_mask != nullptr && p->Gut_s.ord_rows != nullptr && p->Gut_s.ord_nonempty;
   return false;
 }
 
@@ -191,7 +196,7 @@ static int inverse_pass(mlg_plan_s* p, int ax, const float2* y, const float* HY,
   }
   const bool gut_in = fused_gut(p) && ax == d - 1;
   if (gut_in) set_gut_input(p, pd, y, HY);
-  if (run_mode(p) == kAdjMasked && ax == d - 1) {
+  if (adjoint_run_mode(p) == kAdjMasked && ax == d - 1) {
     pd.in_mask = p->Gut_s.nz_mask;
     pd.in_lmask = p->line_mask;
     pd.tmask = p->tmask;
@@ -327,7 +332,7 @@ int nakatsha_stage(mlg_plan_s* p, int stage, const float2* y, const float* HY, f
     a.out.a = p->grid;
     a.out.rows = p->Nu_tot;
     a.long_only = fused_gut(p);
-    a.nonempty_only = run_mode(p) == kAdjMasked;
+    a.nonempty_only = adjoint_run_mode(p) == kAdjMasked;
     a.records = p->gut_records != 0;
     a.unit_count = p->unit_count;
     a.seg_scratch = p->seg_scratch;
@@ -660,7 +665,8 @@ static int plan_create_impl(int imDim, const int* N_u, const int* n_u, int nCh, 
   if ((st = check_gu_covered(p, s)) != MLG_OK) return bail(st);
   p->odd_masked = odd && p->Gut_s.ord_rec && p->Gut_s.ord_short >= 0 && p->tmask;
   p->fwd_masked_store = p->gu_covered ? 1 : 0;
-  p->adjoint_mode = adjoint_mode_valid(p, kAdjMasked) ? kAdjMasked : (imDim >= 2 ? kAdjFused : kAdjFullGrid);
+  p->adjoint_mode = p->odd_masked || adjoint_mode_valid(p, kAdjMasked) ? kAdjMasked
+                                                                        : (imDim >= 2 ? kAdjFused : kAdjFullGrid);
   const size_t kbytes = sizeof(float2) * (size_t)nu * nCh;
   const size_t gbytes = sizeof(float2) * (size_t)Nu * nCh;
   const size_t abytes = sizeof(float2) * (size_t)p->N[0] * p->n[1] * p->n[2] * nCh;

@@ -35,16 +35,17 @@ struct mlg_plan_s {
   //  0 kAdjFullGrid: Gut writes every grid cell, the pass streams the grid;
   //  1 kAdjFused:    the pass gathers Gut rows from k-space itself (2-D/3-D);
   //  2 kAdjMasked:   Gut writes only its non-empty rows, the pass reads a
-  //                  cell only when its occupancy bit is set (even nCh).
+  //                  cell only when its occupancy bit is set (even nCh, or
+  //                  odd_masked with register passes: adjoint_run_mode).
   int adjoint_mode = 0;
+  // Odd coil counts (2-D, 3-D, at most 32) whose matrix and axis have the tables:
+  // with register passes the masked strategy, Gut's non-empty rows a coil per
+  // thread, is theirs too (and the default), and the last forward pass stores
+  // masked where Gu's columns are covered (odd_covered)
+  bool odd_masked = false, odd_covered = false;
   // Gut's occupancy bits regrouped per line of the first inverse pass (axis
   // imDim - 1): line_mask_words words per line (built with the occupancy
   // tables, for kAdjMasked)
-  // Odd coil counts (2-D, 3-D) with register passes: whatever the strategy
-  // set, the adjoint runs as kAdjMasked does for even ones -- Gut's non-empty
-  // rows a coil per thread, occupancy bits in the first pass -- and the last
-  // forward pass stores masked where Gu's columns are covered (odd_covered)
-  bool odd_masked = false, odd_covered = false;
   uint32_t* line_mask = nullptr;
   int line_mask_words = 0;
   // the same bits regrouped for the register passes (PassDesc::tmask; in
@@ -59,12 +60,12 @@ struct mlg_plan_s {
   // forward pass storing only the 32-row chunks that hold cells Gu reads
   // (fwd_masked_store = 1; allowed when gu_covered: every Gu column is an
   // occupied cell of the line masks, checked once at plan creation)
-  // register passes (mlg_fft_reg.cuh; the default) in place of either, for
-  // the pass shapes that have one
-  int reg_passes = 0;
   int pass_buffers = 2;
   int gut_records = 0;
   int fwd_masked_store = 0;
+  // register passes (mlg_fft_reg.cuh; the default) in place of the passes of
+  // pass_buffers, for the pass shapes that have one and do not lose by it
+  int reg_passes = 0;
   bool gu_covered = false;
   cudaStream_t stream = nullptr;  // internal non-blocking stream
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
@@ -116,6 +117,7 @@ int shanna_stage(mlg_plan_s* p, int stage, const float2* x, bool x_per_coil, flo
 int nakatsha_stage(mlg_plan_s* p, int stage, const float2* y, const float* HY, float scale, float2* x,
                    double* partial, int* n_partial, cudaStream_t s);
 bool adjoint_mode_valid(const mlg_plan_s* p, int mode);
+int adjoint_run_mode(const mlg_plan_s* p);
 // whether the plan's passes take bufB in FP16 (mixed CG steps; host check)
 bool half_intermediate_possible(mlg_plan_s* p);
 int shanna_run(mlg_plan_s* p, const float2* x, bool x_per_coil, float2* y, const float* sqn_w, double* partial,

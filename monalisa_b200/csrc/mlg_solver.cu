@@ -528,7 +528,7 @@ extern "C" int mlg_plan_set_adjoint(mlg_plan_t p, int mode) {
 
 extern "C" int mlg_plan_get_adjoint(mlg_plan_t p, int* mode) {
   MLG_CHECK(p && mode, "NULL argument");
-  *mode = p->adjoint_mode;
+  *mode = adjoint_run_mode(p);
   return MLG_OK;
 }
 
@@ -691,7 +691,7 @@ extern "C" int mlg_plan_autotune_variants(mlg_plan_t p, int reps, double* ms) {
   }
   p->reg_passes = best_reg;
   p->fwd_masked_store = best_mask;
-  if (st == MLG_OK && p->Gut_s.ord_rec && p->adjoint_mode == 2) {
+  if (st == MLG_OK && p->Gut_s.ord_rec && p->adjoint_mode == 2 && p->nCh % 2 == 0) {
     double best = 1e30;
     for (int v = 0; v <= 1 && st == MLG_OK; ++v) {
       p->gut_records = v;
@@ -729,7 +729,7 @@ extern "C" int mlg_plan_set_precision(mlg_plan_t p, int precision) {
     MLG_CUDA(cudaStreamSynchronize(p->stream));
   }
   p->precision = precision;
-  if (!adjoint_mode_valid(p, p->adjoint_mode))  // the fused gather reads FP32 k-space
+  if (!adjoint_mode_valid(p, p->adjoint_mode) && !(p->odd_masked && p->adjoint_mode == 2))  // the fused gather reads FP32 k-space
     p->adjoint_mode = adjoint_mode_valid(p, 2) ? 2 : 0;
   if (p->cg_graph) cudaGraphExecDestroy(p->cg_graph);
   p->cg_graph = nullptr;
