@@ -391,12 +391,16 @@ int mlg_plan_autotune_variants(mlg_plan_t p, int reps, double* ms);
  * and cross shared memory once, for the axis lengths that have them
  * (csrc/mlg_fft_reg_lengths.h); other lengths and the fused adjoint's first
  * pass use the passes pass_buffers names.  They agree with those passes up to
- * the rounding of the transforms.  mlg_plan_set_variant turns them off -- the
- * passes it names run -- and this call turns them on again;
- * mlg_plan_autotune_variants times them with the others.  No counterpart in
- * the reference. */
+ * the rounding of the transforms.  mlg_plan_set_variant with another
+ * pass_buffers than the plan's turns them off -- the passes it names run -- and
+ * on again when it names the earlier one, so that the values of
+ * mlg_plan_get_variant restore a plan; this call turns them on or off by name.
+ * mlg_plan_autotune_variants times them with the others
+ * (mlg_plan_get_register_passes_ms: forward + adjoint in milliseconds, negative
+ * when not timed).  No counterpart in the reference. */
 int mlg_plan_set_register_passes(mlg_plan_t p, int on);
 int mlg_plan_get_register_passes(mlg_plan_t p, int* on);
+int mlg_plan_get_register_passes_ms(mlg_plan_t p, double* ms);
 
 /* Precision of the plan's CG-SENSE solver (mlg_sensa_dev / mlg_sensa).
  * MLG_PRECISION_FP32: FP32 data and matrix values, FP64 scalars (the

@@ -57,6 +57,7 @@ SIGNATURES = {
     "mlg_plan_autotune_variants": [c_vp, c_int, P_d],
     "mlg_plan_set_register_passes": [c_vp, c_int],
     "mlg_plan_get_register_passes": [c_vp, P_i],
+    "mlg_plan_get_register_passes_ms": [c_vp, P_d],
     "mlg_plan_set_precision": [c_vp, c_int],
     "mlg_plan_get_precision": [c_vp, P_i],
     "mlg_plan_get_half_intermediate": [c_vp, P_i],

@@ -66,6 +66,10 @@ struct mlg_plan_s {
   // register passes (mlg_fft_reg.cuh; the default) in place of the passes of
   // pass_buffers, for the pass shapes that have one and do not lose by it
   int reg_passes = 0;
+  // the pass_buffers of the plan when naming others turned the register passes
+  // off (mlg_plan_set_variant; -1: on, or turned off by name)
+  int reg_home = -1;
+  double reg_ms = -1.0;           // their time in the last variant tuning
   bool gu_covered = false;
   cudaStream_t stream = nullptr;  // internal non-blocking stream
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;

@@ -583,9 +583,16 @@ extern "C" int mlg_plan_set_variant(mlg_plan_t p, int pass_buffers, int gut_reco
   MLG_CHECK(!gut_records || (p->Gut_s.ord_rec && p->nCh % 2 == 0), "this plan has no Gut row records (masked adjoint, even coil count)");
   MLG_CHECK(!fwd_masked_store || p->gu_covered,
             "this plan cannot mask its forward stores (no line masks, or a Gu column outside Gut's occupied cells)");
-  if (p->reg_passes || p->pass_buffers != pass_buffers || p->gut_records != gut_records ||
-      p->fwd_masked_store != fwd_masked_store) {
-    p->reg_passes = 0;  // the named passes run
+  if (p->pass_buffers != pass_buffers || p->gut_records != gut_records || p->fwd_masked_store != fwd_masked_store) {
+    if (p->pass_buffers != pass_buffers) {
+      if (p->reg_passes) {  // other passes named: they run
+        p->reg_passes = 0;
+        p->reg_home = p->pass_buffers;
+      } else if (pass_buffers == p->reg_home) {  // back to the variant that had them
+        p->reg_passes = 1;
+        p->reg_home = -1;
+      }
+    }
     p->pass_buffers = pass_buffers;
     p->gut_records = gut_records;
     p->fwd_masked_store = fwd_masked_store;
@@ -598,6 +605,7 @@ extern "C" int mlg_plan_set_variant(mlg_plan_t p, int pass_buffers, int gut_reco
 extern "C" int mlg_plan_set_register_passes(mlg_plan_t p, int on) {
   MLG_CHECK(p, "NULL plan");
   MLG_CHECK(on == 0 || on == 1, "register passes: 0 or 1");
+  p->reg_home = -1;
   if (p->reg_passes != on) {
     p->reg_passes = on;
     if (p->cg_graph) cudaGraphExecDestroy(p->cg_graph);  // captured with the other kernels
@@ -612,6 +620,12 @@ extern "C" int mlg_plan_get_register_passes(mlg_plan_t p, int* on) {
   return MLG_OK;
 }
 
+extern "C" int mlg_plan_get_register_passes_ms(mlg_plan_t p, double* ms) {
+  MLG_CHECK(p && ms, "NULL argument");
+  *ms = p->reg_ms;
+  return MLG_OK;
+}
+
 extern "C" int mlg_plan_get_variant(mlg_plan_t p, int* pass_buffers, int* gut_records, int* fwd_masked_store) {
   MLG_CHECK(p && pass_buffers && gut_records && fwd_masked_store, "NULL argument");
   *pass_buffers = p->pass_buffers;
@@ -621,11 +635,11 @@ extern "C" int mlg_plan_get_variant(mlg_plan_t p, int* pass_buffers, int* gut_re
 }
 
 // Times the kernel variants of the plan's current adjoint strategy and keeps
-// the fastest (the register passes included): ms[0..2] = forward + adjoint with TMA passes over 2 / 3
-// buffers and with cp.async passes (masked forward stores where the plan
-// allows them), ms[3..4] = adjoint with Gut from the CSR / from row records,
-// ms[5] = forward + adjoint storing every chunk of the grid, at the chosen
-// buffer count (-1: not available).
+// the fastest (the register passes included, their time in reg_ms): ms[0..2] =
+// forward + adjoint with TMA passes over 2 / 3 buffers and with cp.async passes
+// (masked forward stores where the plan allows them), ms[3..4] = adjoint with Gut
+// from the CSR / from row records, ms[5] = forward + adjoint storing every chunk
+// of the grid, at the chosen buffer count (-1: not available).
 extern "C" int mlg_plan_autotune_variants(mlg_plan_t p, int reps, double* ms) {
   using namespace mlg;
   MLG_CHECK(p && reps >= 1, "invalid argument");
@@ -683,10 +697,12 @@ extern "C" int mlg_plan_autotune_variants(mlg_plan_t p, int reps, double* ms) {
   // the register passes (whole-grid stores never beat masked ones there)
   // against the best of the above
   int best_reg = reg0;
+  double reg_ms = -1.0;
   if (st == MLG_OK && best_fwd > 0.0) {
     p->reg_passes = 1;
     p->fwd_masked_store = p->gu_covered ? 1 : 0;
-    best_reg = time_it(true) < (t[5] > 0.0 ? std::min(best_fwd, t[5]) : best_fwd) ? 1 : 0;
+    reg_ms = time_it(true);
+    best_reg = reg_ms < (t[5] > 0.0 ? std::min(best_fwd, t[5]) : best_fwd) ? 1 : 0;
     if (best_reg) best_mask = p->fwd_masked_store;
   }
   p->reg_passes = best_reg;
@@ -706,6 +722,7 @@ extern "C" int mlg_plan_autotune_variants(mlg_plan_t p, int reps, double* ms) {
   p->gut_records = rec0;
   p->fwd_masked_store = mask0;
   p->reg_passes = reg0;
+  p->reg_ms = reg_ms;
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   if (ms)

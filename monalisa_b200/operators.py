@@ -230,9 +230,9 @@ class NufftPlan:
 
     def autotune(self, reps: int = 3, variants: bool = True) -> dict:
         """Times the valid adjoint strategies and keeps the fastest, then (with
-        `variants`) the kernel variants of that strategy (TMA or cp.async
-        line-FFT passes, Gut rows from the CSR or from row records); returns
-        {name: ms} (what the plan cannot run is omitted)."""
+        `variants`) the kernel variants of that strategy (register, TMA or
+        cp.async line-FFT passes, Gut rows from the CSR or from row records);
+        returns {name: ms} (what the plan cannot run is omitted)."""
         ms = np.zeros(3)
         N.call("mlg_plan_autotune", self._h, int(reps), N.dptr(ms))
         out = {n: float(t) for n, t in zip(self.ADJOINT_MODES, ms) if t >= 0}
@@ -242,6 +242,10 @@ class NufftPlan:
             names = ("passes_tma_2buf", "passes_tma_3buf", "passes_cp_async", "gut_csr", "gut_records",
                      "fwd_full_store")
             out.update({n: float(t) for n, t in zip(names, mv) if t >= 0})
+            reg = ctypes.c_double()
+            N.call("mlg_plan_get_register_passes_ms", self._h, ctypes.byref(reg))
+            if reg.value >= 0:
+                out["passes_register"] = reg.value
         return out
 
     @property
