@@ -424,8 +424,10 @@ int mlg_plan_get_precision(mlg_plan_t p, int* precision);
 /* *on != 0 when a mixed solve of this plan keeps the intermediate of its
  * 3-D transforms (after the forward y pass, after the adjoint z pass) in
  * scaled FP16 inside the CG steps: MLG_PRECISION_MIXED, 3-D, a multiple of 4
- * coils, no fused adjoint gather, and TMA or register line passes for those
- * shapes (bit 0); bit 1 set when the forward grid is stored in scaled FP16 as
+ * coils, no fused adjoint gather, and pass shapes that the TMA line passes take
+ * with the plan's pass_buffers (axis lengths 2^k and 3 * 2^k; bit 0) -- also where
+ * the register passes run, which would load and store FP16 at other shapes: those
+ * keep FP32; bit 1 set when the forward grid is stored in scaled FP16 as
  * well (the last forward pass writes it, Gu's gathers read it: even coil count,
  * no Gu row longer than 256 entries); 0 otherwise.  No reference counterpart. */
 int mlg_plan_get_half_intermediate(mlg_plan_t p, int* on);

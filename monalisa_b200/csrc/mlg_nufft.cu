@@ -252,7 +252,9 @@ static int inverse_pass(mlg_plan_s* p, int ax, const float2* y, const float* HY,
 
 // Whether the CG steps of a mixed solve keep bufB in FP16: a 3-D plan, a
 // coil count whose FP16 cells fill 16-byte TMA rows, no fused Gut gather (it
-// reads FP32), and a dry run of the four passes accepted by their kernels.
+// reads FP32), and a dry run of the four passes accepted by the TMA kernels (the
+// register passes, where they run instead, take every such shape, and others that
+// keep FP32).
 // Cached per (pass_buffers, adjoint_mode), the plan state the pass kernels
 // depend on.
 bool half_intermediate_possible(mlg_plan_s* p) {

@@ -214,8 +214,9 @@ class NufftPlan:
     def half_intermediate(self) -> bool:
         """Whether the CG steps of a mixed solve keep the intermediate of the
         3-D transforms (after the y pass of the forward, the z pass of the
-        adjoint) in scaled FP16: mixed precision on a plan whose passes support
-        it (3-D, a multiple of 4 coils, TMA or register line passes)."""
+        adjoint) in scaled FP16: mixed precision on a plan whose shapes the TMA
+        line passes take (3-D, a multiple of 4 coils, axis lengths 2^k and
+        3 * 2^k, 'pass_buffers' 2 or 3), whichever passes run."""
         m = ctypes.c_int()
         N.call("mlg_plan_get_half_intermediate", self._h, ctypes.byref(m))
         return bool(m.value & 1)
