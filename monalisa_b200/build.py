@@ -64,7 +64,8 @@ def build(verbose: bool = False, jobs: int | None = None) -> str:
     os.makedirs(LIB, exist_ok=True)
     os.makedirs(os.path.join(LIB, "mex"), exist_ok=True)
     os.makedirs(OBJ, exist_ok=True)
-    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(INCLUDE, "*.h"))
+    headers = [h for pat in (os.path.join(CSRC, "*.cuh"), os.path.join(CSRC, "*.h"), os.path.join(INCLUDE, "*.h"))
+               for h in glob.glob(pat)]
     cu = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
     cpp = sorted(glob.glob(os.path.join(CSRC, "*.cpp")))
     so = os.path.join(LIB, "libmonalisa_gpu.so")
