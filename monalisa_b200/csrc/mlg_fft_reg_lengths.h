@@ -1,7 +1,22 @@
 // The axis lengths with register passes, N = A * B (A a multiple of 4, both at
 // most 32), in groups of about equal compile time (one translation unit
-// each).  X(N, A, B, MAIN): MAIN lengths have kernels specialised for twofold
-// oversampling too.
+// each).  In: the lengths from 16 to 768 with prime factors up to 7 that split so
+// (20, 28 and 36 aside), and 800, 896, 960 and 1024.  784, 840 and 864 would split
+// too and are not built; lengths with factors 11 and 13 (176, 208, 352, 416) have
+// no sub-transforms here: they run the direct DFT, as all but 2^k and 3 * 2^k did.
+// Against the shared-memory passes (sum of the passes of a forward and an adjoint,
+// us, twofold oversampling): 16^3 x 8 coils 45 / 46, 32^3 x 16 50 / 53, 48^3 x 8 49
+// / 55, 512^2 x 12 64 / 125, 768^2 x 8 84 / 126, 1024^2 x 4 80 / 178; 96 to 192
+// points: shared_pass_faster in mlg_fft.cu.
+//
+// X(N, A, B, MAIN): MAIN lengths have kernels specialised for twofold
+// oversampling and, with sub-transforms of up to 16 points, two columns per thread
+// too, for three times the kernels: the grids of the matrix sizes most in use (32
+// to 64 in steps of 8, 72 to 256; no rule on the length's factors).  What
+// the others lose in 3-D, ps per grid value over the six passes, 8 coils: 108 13.5,
+// 168 9.3, 180 9.1, 200 12.0, 216 10.8 beside 112 11.1, 160 8.3, 192 7.2, 224 6.6;
+// long sub-transforms more (140 15.8, 196 20.3, 252 14.4).  In 2-D nothing to 5 %
+// (a launch's latency each: 336^2 x 8 coils 52.7, 320^2 52.6, 420^2 38.2, 400^2 36.1).
 #pragma once
 
 #define MLG_REG_GROUP_0(X) \
